@@ -9,9 +9,15 @@
 
 namespace fq {
 
-template <typename WT, bool PHI, int SC, int GM, int GM2, bool TURN = false, bool ST = true>
+template <typename WT, bool PHI, int SC, int GM, int GM2, bool TURN = false, bool ST = true,
+          bool MIR = false>
 inline int dual_launch(fq_ctx* ctx, const PassArgs& A, double* gb, double* gg, double* gb2) {
-    auto fn = k_pass_dual<WT, PHI, SC, ST, GM, GM2, TURN>;
+    if constexpr (SC == SC_L021 && !MIR) {
+        if (A.mir)
+            return dual_launch<WT, PHI, SC, GM, GM2, TURN, ST, true>(ctx, A, gb, gg, gb2);
+    }
+    FQ_CHECK(MIR || !A.mir, FQ_ERR_INVALID, "this adjoint pass has no mirror form");
+    auto fn = k_pass_dual<WT, PHI, SC, ST, GM, GM2, TURN, MIR>;
     FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)dual_smem_bytes<WT>(kMaxQubits)));
     const i64 grid = std::min<i64>(A.ntiles, (i64)ctx->num_sms);
@@ -19,7 +25,7 @@ inline int dual_launch(fq_ctx* ctx, const PassArgs& A, double* gb, double* gg, d
     fn<<<(unsigned)grid, kPassThreads, dual_smem_bytes<WT>(A.N), ctx->stream>>>(A, gb, gg, gb2);
     FQ_CUDA(cudaGetLastError());
     // The turnaround reads one vector and writes two; ST = false reads two.
-    prof_end(ctx, tok, FQ_KIND_ADJOINT, (TURN ? 48.0 : ST ? 64.0 : 32.0) * (double)(1ull << A.N));
+    prof_end(ctx, tok, FQ_KIND_ADJOINT, (TURN ? 48.0 : ST ? 64.0 : 32.0) * (double)A.ntiles * kTile);
     ctx->launches++;
     return FQ_OK;
 }

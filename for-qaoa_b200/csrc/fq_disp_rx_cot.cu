@@ -1,13 +1,18 @@
 // fq_disp_rx_cot.cu -- strided RX passes of the fused engine with the
-// reduced gate [[u,-i],[-i,u]], u = cot(beta/2), optionally accumulating <C>.
+// reduced gate [[u,-i],[-i,u]], u = cot(beta/2), for a circuit's last
+// pass writing both halves of the state and optionally accumulating <C>.
 #include "fq_launch.cuh"
 
 namespace fq {
 
 int dispatch_rx_cot(fq_ctx* ctx, bool integer, bool energy, const PassArgs& A) {
-    if (!energy) return launch_pass<int, PH_NONE, GM_COT, EX_NONE, true>(ctx, A);
-    if (integer) return launch_pass<int, PH_NONE, GM_COT, EX_ENERGY, true>(ctx, A);
-    return launch_pass<double, PH_NONE, GM_COT, EX_ENERGY, true>(ctx, A);
+    if (!A.full) {
+        FQ_CHECK(!energy, FQ_ERR_INVALID, "<C> belongs to a circuit's last pass");
+        return launch_pass<int, PH_NONE, GM_COT, EX_NONE, 1>(ctx, A);
+    }
+    if (!energy) return launch_pass<int, PH_NONE, GM_COT, EX_NONE, 2>(ctx, A);
+    if (integer) return launch_pass<int, PH_NONE, GM_COT, EX_ENERGY, 2>(ctx, A);
+    return launch_pass<double, PH_NONE, GM_COT, EX_ENERGY, 2>(ctx, A);
 }
 
 }  // namespace fq

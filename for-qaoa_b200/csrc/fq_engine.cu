@@ -221,12 +221,18 @@ static int choose_lrows(int N) {
 // passes over the highest qubits lead and the one over the lowest closes
 // each layer: an odd circuit then ends on the faster of the two strided
 // geometries (61.2-61.8 against 60.3-61.0 layers/s, A/B in one call).
-std::vector<PassPlan> plan_layer(int N) {
+// A half state's passes cover the same number of qubits: the mirror tile
+// takes qubits 0..10 and N-1, the strided ones 11..N-2.
+std::vector<PassPlan> plan_layer(int N, bool half) {
     std::vector<PassPlan> v;
-    v.push_back({kTileBits, kTileBits, (1u << kTileBits) - 1});
+    if (half)
+        v.push_back({kTileBits - 1, N - 1, (1u << kTileBits) - 1, 1});
+    else
+        v.push_back({kTileBits, kTileBits, (1u << kTileBits) - 1});
     const int lrows = choose_lrows(N);
-    for (int q = kTileBits; q < N;) {
-        const int k = std::min(kTileBits - lrows, N - q);
+    const int end = half ? N - 1 : N;
+    for (int q = half ? kTileBits - 1 : kTileBits; q < end;) {
+        const int k = std::min(kTileBits - lrows, end - q);
         const int l = kTileBits - k;
         v.push_back({l, q, ((1u << k) - 1) << l});
         q += k;
@@ -284,6 +290,16 @@ PassArgs base_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g) {
     A.scale = 1.0;
     A.pf_dist = prefetch_distance();
     A.err = ctx->d_err;
+    return A;
+}
+
+PassArgs engine_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g, const PassPlan& p) {
+    PassArgs A = base_args(ctx, sv, N, g);
+    if (half_state(N)) A.ntiles >>= 1;
+    A.l = p.l;
+    A.a = p.a;
+    A.tmask = p.tmask;
+    A.mir = p.mir;
     return A;
 }
 
@@ -415,7 +431,7 @@ static int tile_cut_tables(fq_ctx* ctx, const GraphPrep& g, int N,
     tabs.assign(plan.size(), nullptr);
     if (N < 21 || plan.size() > 4) return FQ_OK;
     const size_t wt = g.integer ? sizeof(int) : sizeof(double);
-    const i64 ntiles = 1ll << (N - kTileBits);
+    const i64 ntiles = 1ll << (N - kTileBits - 1);  // a half state's
     const size_t per = (size_t)ntiles * kTcutStride * wt;
     const size_t need = per * plan.size();
     // Built for these weights (no upload since) and this N: reuse them, as
@@ -521,10 +537,7 @@ static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const Graph
         for (int j = (p == 0 ? 0 : 1); j < npass; j++) {
             if (skip_last && p == P - 1 && j == npass - 1) break;
             const int idx = (p % 2 == 0) ? j : npass - 1 - j;
-            PassArgs A = base_args(ctx, sv, N, g);
-            A.l = plan[idx].l;
-            A.a = plan[idx].a;
-            A.tmask = plan[idx].tmask;
+            PassArgs A = engine_args(ctx, sv, N, g, plan[idx]);
             A.tcut = tcut[idx];
             A.gx = gx[p];
             const bool last_of_layer = j == npass - 1;
@@ -539,7 +552,8 @@ static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const Graph
                 ph = PH_MUL;
                 FQ_TRY(dispatch_fused(ctx, g.integer, gm[p], gm[p + 1], A));
             } else {
-                const bool ex = energy && p == P - 1 && last_of_layer;
+                A.full = p == P - 1 && last_of_layer;
+                const bool ex = energy && A.full;
                 FQ_TRY(dispatch_rx(ctx, g.integer, gm[p], ex, A));
             }
             last_grid = pass_grid(ctx, A, ph, true);
@@ -549,19 +563,19 @@ static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const Graph
 }
 
 bool engine_fused(const GraphPrep& g, int N, int P) {
-    return fuse_enabled() && plan_layer(N).size() >= 2 && P >= 2 &&
+    return fuse_enabled() && half_state(N) && P >= 2 &&
            (!g.integer || (engine_nhi(g) > 0 && P <= kMaxTableLayers));
 }
 
 int engine_last_pass(const GraphPrep& g, int N, int P) {
-    const int npass = (int)plan_layer(N).size();
+    const int npass = (int)plan_layer(N, half_state(N)).size();
     return (engine_fused(g, N, P) && (P - 1) % 2 == 1) ? 0 : npass - 1;
 }
 
 int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, const double* gammas,
                    const double* betas, double* energy, bool skip_last) {
     const double amp0 = fq_init_amp(N);
-    const std::vector<PassPlan> plan = plan_layer(N);
+    const std::vector<PassPlan> plan = plan_layer(N, half_state(N));
     int last_grid = 0;
     const bool fused = engine_fused(g, N, P);
     FQ_CHECK(!(skip_last && (energy || plan.size() < 2)), FQ_ERR_INVALID,
@@ -593,10 +607,8 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
         }
         for (size_t i = 0; i < plan.size(); i++) {
             if (skip_last && p == P - 1 && i + 1 == plan.size()) break;
-            PassArgs A = base_args(ctx, sv, N, g);
-            A.l = plan[i].l;
-            A.a = plan[i].a;
-            A.tmask = plan[i].tmask;
+            PassArgs A = engine_args(ctx, sv, N, g, plan[i]);
+            A.full = half_state(N) && p == P - 1 && i + 1 == plan.size();
             A.tcut = tcut[i];
             A.gx = gx;
             if (nhi > 0) set_table_args(A, g, gammas[p], scale);
@@ -621,6 +633,7 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
         }
         FQ_TRY(reduce_to_result(ctx, last_grid));
         FQ_TRY(read_result(ctx, energy));
+        if (half_state(N)) *energy *= 2.0;  // the swept half's sum
     }
     return FQ_OK;
 }

@@ -11,16 +11,30 @@
 namespace fq {
 
 // One pass of a layer: tile bits 0..l-1 = physical 0..l-1, tile bits
-// l..11 = physical a..a+11-l, RX on the tile bits of tmask.
+// l..11 = physical a..a+11-l, RX on the tile bits of tmask; mir: the mirror
+// pass of a half state (fq_pass.cuh).
 struct PassPlan {
     int l, a;
     unsigned tmask;
+    int mir = 0;
 };
 
 // Passes of one layer for N >= 12: the contiguous tile over qubits 0..11
 // and strided tiles over the remaining qubits (the first strided one leads
 // when there are three or more passes); the first pass carries the phase.
-std::vector<PassPlan> plan_layer(int N);
+// half (N >= 13): the passes of a half state, the mirror tile over qubits
+// 0..10 and N-1 and strided tiles over qubits 11..N-2.
+std::vector<PassPlan> plan_layer(int N, bool half = false);
+// Whether whole circuits from |+>^N run on a half state (fq_pass.cuh): every
+// N whose half fills a tile.  The passes are bound by on-chip work and HBM
+// traffic per amplitude, and both halve.  On B200, against sweeping the
+// whole state (A/B in one call): forward N=30 p=5 40.0 against 77.6 ms, N=28
+// p=3 with FP64 weights 6.20 against 11.87 ms, N=23 p=4 0.315 against
+// 0.493 ms; gradient N=26 p=10 15.5 against 30.7 ms.  At N <= 20 the
+// passes' set-up and latency dominate: forward N=20 p=5 140 against 164 us.
+inline bool half_state(int N) { return N > kTileBits; }
+// Pass arguments of plan entry p on the engine's state (half for N >= 13).
+PassArgs engine_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g, const PassPlan& p);
 // Reduced RX for angle beta: gate mode, t or u, and the factor f.
 void gate_params(double beta, int& gm, double& g, double& f);
 PassArgs base_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g);

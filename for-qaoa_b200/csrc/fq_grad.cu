@@ -185,7 +185,8 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     FQ_CHECK(sv != costate, FQ_ERR_INVALID, "state and costate must be different buffers");
     GraphPrep g;
     FQ_TRY(setup_graph(ctx, graph, N, g));
-    const std::vector<PassPlan> plan = plan_layer(N);
+    const bool half = half_state(N);
+    const std::vector<PassPlan> plan = plan_layer(N, half);
     const int npass = (int)plan.size();
     FQ_CHECK(1 + P + P * npass < kResultWords, FQ_ERR_INVALID, "P=%d too large", P);
 
@@ -225,12 +226,14 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     FQ_TRY(engine_forward(ctx, sv, N, P, g, gammas, betas, nullptr, turn));
     if (!turn) {
         PassArgs A = base_args(ctx, sv, N, g);
+        if (half) A.ntiles >>= 1;
         A.sv2 = (double2*)costate;
         FQ_TRY(dispatch_costate(ctx, g.integer, A));
         FQ_TRY(reduce_partials(ctx, ctx->d_partial, pass_grid(ctx, A, PH_NONE, false),
                                ctx->d_result));
     }
-    const int grid = (int)std::min<i64>(1ll << (N - kTileBits), (i64)ctx->num_sms);
+    const int grid =
+        (int)std::min<i64>(1ll << (N - kTileBits - (half ? 1 : 0)), (i64)ctx->num_sms);
     const bool batched = (i64)nrev * 3 * grid <= ctx->partial_cap && 3 * nrev <= kMaxGradSums;
     const bool all_tables = g.integer && engine_nhi(g) > 0 && P <= kMaxTableLayers;
     const int nhi = g.integer ? engine_nhi(g) : 0;
@@ -243,11 +246,8 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     for (int q = 0; q < nrev; q++) {
         const RevPass& R = rev[q];
         const int k = R.k, i = R.i;
-        PassArgs A = base_args(ctx, sv, N, g);
+        PassArgs A = engine_args(ctx, sv, N, g, plan[i]);
         A.sv2 = (double2*)costate;
-        A.l = plan[i].l;
-        A.a = plan[i].a;
-        A.tmask = plan[i].tmask;
         const int nt = __builtin_popcount(plan[i].tmask);
         A.gx = gx[k];
         A.f2 = f[k] * f[k];
@@ -324,7 +324,9 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
 
 int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,
                  double* grad_beta) {
-    const int npass = (int)plan_layer(N).size();
+    const bool half = half_state(N);
+    const double m = half ? 2.0 : 1.0;  // the sums of a half state are half the whole
+    const int npass = (int)plan_layer(N, half).size();
     const double* r = ctx->h_result;
     int flag = 0;
     memcpy(&flag, r + kResultWords - 1, sizeof(int));
@@ -333,12 +335,12 @@ int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,
         set_error("a device-side bounded wait gave up (flag %d); results are incomplete", flag);
         return FQ_ERR_TIMEOUT;
     }
-    *energy = r[0];
+    *energy = m * r[0];
     for (int k = 0; k < P; k++) {
-        grad_gamma[k] = -r[1 + k];
+        grad_gamma[k] = -m * r[1 + k];
         double s = 0;
         for (int i = 0; i < npass; i++) s += r[1 + P + k * npass + i];
-        grad_beta[k] = s;
+        grad_beta[k] = m * s;
     }
     return FQ_OK;
 }

@@ -17,7 +17,7 @@
 namespace fq {
 
 // Kind of a pass for profiling, and the HBM bytes it must move.
-template <int PH, int GM, int EX, bool ST>
+template <int PH, int GM, int EX, int ST>
 inline int pass_kind() {
     if ((EX == EX_ENERGY || EX == EX_COSTATE) && !ST) return FQ_KIND_EXPECT;
     if (EX == EX_DIAG) return FQ_KIND_EXPECT;
@@ -27,11 +27,11 @@ inline int pass_kind() {
     return PH != PH_NONE ? FQ_KIND_PHASE_PASS : FQ_KIND_MIXER_PASS;
 }
 
-template <int PH, int EX, bool ST>
-inline double pass_bytes(int N) {
-    const double n = (double)(1ull << N);
+template <int PH, int EX, int ST>
+inline double pass_bytes(const PassArgs& A) {
+    const double n = (double)A.ntiles * kTile;
     const bool load = (PH != PH_INIT) && (ST || EX == EX_ENERGY || EX == EX_COSTATE);
-    return n * ((load ? 16.0 : 0.0) + (ST ? 16.0 : 0.0) + (EX == EX_DIAG ? 8.0 : 0.0) +
+    return n * ((load ? 16.0 : 0.0) + 16.0 * ST + (EX == EX_DIAG ? 8.0 : 0.0) +
                 (EX == EX_COSTATE ? 16.0 : 0.0));
 }
 
@@ -46,10 +46,10 @@ inline double pass_bytes(int N) {
 // against 242 ms per N=32 circuit (p=3), A/B in one call.
 inline bool pair_ok(const PassArgs& A) { return A.l >= 1 && A.l <= 3 && A.a > A.l && A.ntiles >= 2; }
 
-template <typename WT, int PH, int GM, int EX, bool ST, int SC, int GM2 = GM_NONE,
-          bool PAIR = false>
+template <typename WT, int PH, int GM, int EX, int ST, int SC, int GM2 = GM_NONE,
+          bool PAIR = false, bool MIR = false>
 inline int launch_ldg_as(fq_ctx* ctx, const PassArgs& A) {
-    auto fn = k_pass<WT, PH, GM, EX, ST, SC, GM2, PAIR>;
+    auto fn = k_pass<WT, PH, GM, EX, ST, SC, GM2, PAIR, MIR>;
     const size_t smem = pass_smem_bytes<WT>(A.N, PAIR);
     FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const i64 units = PAIR ? A.ntiles / 2 : A.ntiles;
@@ -58,13 +58,18 @@ inline int launch_ldg_as(fq_ctx* ctx, const PassArgs& A) {
     fn<<<(unsigned)grid, PAIR ? 2 * kPassThreads : kPassThreads, smem, ctx->stream>>>(A);
     FQ_CUDA(cudaGetLastError());
     ctx->last_grid = (int)grid;
-    prof_end(ctx, tok, pass_kind<PH, GM, EX, ST>(), pass_bytes<PH, EX, ST>(A.N));
+    prof_end(ctx, tok, pass_kind<PH, GM, EX, ST>(), pass_bytes<PH, EX, ST>(A));
     ctx->launches++;
     return FQ_OK;
 }
 
-template <typename WT, int PH, int GM, int EX, bool ST, int SC, int GM2 = GM_NONE>
+template <typename WT, int PH, int GM, int EX, int ST, int SC, int GM2 = GM_NONE>
 inline int launch_ldg(fq_ctx* ctx, const PassArgs& A) {
+    if constexpr (SC == SC_L021 && GM != GM_NONE && GM != GM_FULL &&
+                  (EX == EX_NONE || EX == EX_ENERGY)) {
+        if (A.mir) return launch_ldg_as<WT, PH, GM, EX, ST, SC, GM2, false, true>(ctx, A);
+    }
+    FQ_CHECK(!A.mir, FQ_ERR_INVALID, "this pass has no mirror form");
     if (pair_ok(A)) return launch_ldg_as<WT, PH, GM, EX, ST, SC, GM2, true>(ctx, A);
     return launch_ldg_as<WT, PH, GM, EX, ST, SC, GM2, false>(ctx, A);
 }
@@ -93,7 +98,7 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
 // contiguous RX pass: 6.0 ms against 6.9 ms on the TMA pipeline); passes
 // with a phase always do.
 inline bool tma_for(int ph, const PassArgs& A) {
-    return ph == PH_NONE && A.l >= 4 && A.l < kTileBits;
+    return ph == PH_NONE && A.l >= 4 && A.l < kTileBits && !A.mir;
 }
 
 // The state as a tensor of float64 whose innermost dimension is one 128-byte
@@ -142,17 +147,17 @@ inline bool make_pass_tmap(const PassArgs& A, CUtensorMap* map, TmaGeom* G) {
     return r == CUDA_SUCCESS;
 }
 
-template <typename WT, int PH, int GM, int EX, int SC>
+template <typename WT, int PH, int GM, int EX, int ST, int SC>
 inline int launch_tma(fq_ctx* ctx, const PassArgs& A, const CUtensorMap& map, TmaGeom G) {
     const i64 grid = std::min<i64>(A.ntiles, (i64)ctx->num_sms);
     const int tok = prof_begin(ctx);
-    auto fn = k_pass_tma<WT, PH, GM, EX, SC>;
+    auto fn = k_pass_tma<WT, PH, GM, EX, ST, SC>;
     FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)tma_pass_smem_bytes<WT>(kMaxQubits)));
     fn<<<(unsigned)grid, kPassThreads, tma_pass_smem_bytes<WT>(A.N), ctx->stream>>>(A, map, G);
     FQ_CUDA(cudaGetLastError());
     ctx->last_grid = (int)grid;
-    prof_end(ctx, tok, pass_kind<PH, GM, EX, true>(), pass_bytes<PH, EX, true>(A.N));
+    prof_end(ctx, tok, pass_kind<PH, GM, EX, ST>(), pass_bytes<PH, EX, ST>(A));
     ctx->launches++;
     return FQ_OK;
 }
@@ -161,7 +166,7 @@ inline int launch_tma(fq_ctx* ctx, const PassArgs& A, const CUtensorMap& map, Tm
 // without RX (cost phase, <C>, cut diagonal) use the L0 schedule.  RX passes
 // that read and write the state run as TMA pipelines where tma_for() and
 // the tile geometry allow; every other pass uses k_pass.
-template <typename WT, int PH, int GM, int EX, bool ST>
+template <typename WT, int PH, int GM, int EX, int ST>
 inline int launch_pass(fq_ctx* ctx, const PassArgs& A) {
     if constexpr (ST && PH != PH_INIT && EX != EX_DIAG && EX != EX_COSTATE) {
         if (tma_for(PH, A)) {
@@ -169,12 +174,12 @@ inline int launch_pass(fq_ctx* ctx, const PassArgs& A) {
             TmaGeom G;
             if (make_pass_tmap(A, &map, &G)) {
                 if constexpr (GM == GM_NONE) {
-                    return launch_tma<WT, PH, GM, EX, SC_L0>(ctx, A, map, G);
+                    return launch_tma<WT, PH, GM, EX, ST, SC_L0>(ctx, A, map, G);
                 } else {
                     switch (schedule_for(A.tmask)) {
-                        case SC_L021: return launch_tma<WT, PH, GM, EX, SC_L021>(ctx, A, map, G);
-                        case SC_L01: return launch_tma<WT, PH, GM, EX, SC_L01>(ctx, A, map, G);
-                        default: return launch_tma<WT, PH, GM, EX, SC_L0>(ctx, A, map, G);
+                        case SC_L021: return launch_tma<WT, PH, GM, EX, ST, SC_L021>(ctx, A, map, G);
+                        case SC_L01: return launch_tma<WT, PH, GM, EX, ST, SC_L01>(ctx, A, map, G);
+                        default: return launch_tma<WT, PH, GM, EX, ST, SC_L0>(ctx, A, map, G);
                     }
                 }
             }
@@ -199,7 +204,8 @@ inline int pass_grid(fq_ctx* ctx, const PassArgs&, int, bool) { return ctx->last
 // Layer pass with a cost phase (ph = PH_INIT or PH_MUL) and RX on A.tmask
 // (gm = GM_TAN or GM_COT), or the cost phase alone (gm = GM_NONE).
 int dispatch_phase_pass(fq_ctx* ctx, bool integer, int ph, int gm, const PassArgs& A);
-// RX on A.tmask without a phase (reduced gates), optionally with <C>.
+// RX on A.tmask without a phase (reduced gates); with A.full (a forward
+// circuit's last pass) both halves are written, optionally with <C>.
 int dispatch_rx_tan(fq_ctx* ctx, bool integer, bool energy, const PassArgs& A);
 int dispatch_rx_cot(fq_ctx* ctx, bool integer, bool energy, const PassArgs& A);
 // RX with the full formula of src/rx.cu:47-50 (reference-path kernels).

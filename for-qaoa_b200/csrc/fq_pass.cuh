@@ -31,6 +31,20 @@
 // (those bits are lane bits in L0 and L1), so a strided pass with 128-byte
 // rows (9 qubits, tile bits 3..11) also needs one exchange.
 //
+// Half states.  A circuit from |+>^N keeps psi(~z) = psi(z): the start, the
+// cut phase (C(~z) = C(z)) and RX on every qubit commute with flipping all
+// bits, and so does lambda = C psi.  The engine's circuits and gradients of
+// N >= 13 qubits therefore sweep only the 2^(N-1) amplitudes with qubit N-1
+// = 0, half the traffic and half the arithmetic.  An amplitude z with qubit
+// N-1 set is stored at ~z.  Strided tiles over qubits 11..N-2 are those of
+// the whole state with that bit 0; the contiguous pass becomes the mirror
+// pass (MIR): tile bits 0..10 are physical bits 0..10 and tile bit 11 is
+// qubit N-1, i.e. l = 11, a = N-1, with the upper half of each tile at the
+// mirrored addresses 2^(N-1) - 1 - x (two runs of 2048 contiguous
+// amplitudes, one walked backwards).  Phases, cut constants and rotations
+// see an ordinary tile of the N-qubit state.  The pass that ends a forward
+// circuit writes both halves (ST = 2).  Measured: half_state, fq_engine.h.
+//
 // Cut value of an amplitude (exact in integers for integer weights):
 //   C(z) = K(fixed) + C_TT(tile bits) + sum_{u in tile} z_u e_u(fixed)
 // with K = cut inside the fixed bits + sum_m z_m D_m, D_m = sum_{u in tile}
@@ -112,6 +126,8 @@ struct PassArgs {
     // own (CutTables::tile, warps 0 and 1, then a barrier).
     const void* tcut;
     int* err;        // device error flag (bounded waits that gave up)
+    int mir;         // mirror pass of a half state (k_pass, k_pass_dual with MIR)
+    int full;        // write both halves of the state (ST = 2)
 };
 
 __device__ __forceinline__ int tile_phys(int j, int l, int a) { return j < l ? j : a + j - l; }
@@ -701,10 +717,17 @@ __device__ __forceinline__ double2 phase_of(const PassArgs& A, const double2* sm
 // barrier.  Their loads and stores then meet DRAM as rows twice as long
 // (256 bytes at l = 3): per-thread sweeps over 128-byte rows measured
 // 4.1-4.9 TB/s on B200 at N=30, over 256-byte rows 5.6 TB/s.
-template <typename WT, int PH, int GM, int EX, bool ST, int SC, int GM2 = GM_NONE,
-          bool PAIR = false>
+//
+// ST: 0 leaves the state unwritten, 1 writes it back, 2 writes both halves
+// from a half state (each amplitude x of the lower half also at 2^N - 1 - x).
+// MIR: the mirror pass of a half state (see the header comment).
+template <typename WT, int PH, int GM, int EX, int ST, int SC, int GM2 = GM_NONE,
+          bool PAIR = false, bool MIR = false>
 __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ? 1 : 2)
     k_pass(const PassArgs A) {
+    static_assert(!(MIR && PAIR), "mirror tiles are contiguous runs: not paired");
+    static_assert(!MIR || SC == SC_L021, "a mirror pass rotates tile bits 0..11");
+    static_assert(!MIR || EX == EX_NONE || EX == EX_ENERGY, "no costate or diagonal here");
     extern __shared__ __align__(16) unsigned char smraw[];
     using SM = PassSmem<WT>;
     const int grp = PAIR ? (int)(threadIdx.x >> 8) : 0;  // the thread's group (tile of the pair)
@@ -751,6 +774,10 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
     const i64 s10 = 1ll << tile_phys(10, l, a), s11 = 1ll << tile_phys(11, l, a);
     const i64 s4 = 1ll << tile_phys(4, l, a), s5 = 1ll << tile_phys(5, l, a);
     const i64 s6 = 1ll << tile_phys(6, l, a), s7 = 1ll << tile_phys(7, l, a);
+    // Mirror pass: element (b, t) of a tile, b = tile bit 11, is stored at
+    // base + t (b = 0) or mtop - base - t (b = 1); the whole state's index of
+    // the other half is mfull minus a stored index.
+    const i64 mtop = (1ll << (N - 1)) - 1, mfull = (1ll << N) - 1;
     auto off0 = [&](int r) -> i64 {
         return ((r & 1) ? s8 : 0) + ((r & 2) ? s9 : 0) + ((r & 4) ? s10 : 0) + ((r & 8) ? s11 : 0);
     };
@@ -763,6 +790,97 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
     // (SC_L021), a single one is rotated by shuffles in L0.
     const int lo_lane = (SC != SC_L021 && m_lo) ? __ffs(m_lo) - 1 : -1;
     double acc = 0, comp = 0;  // Kahan-compensated <C> accumulator
+    // Loads and stores of a thread's 16 amplitudes of the tile at `base` in
+    // layouts L0 and L1.  A mirror tile's L0 registers 8..15 and L1 warps
+    // 4..7 hold tile bit 11 set.
+    auto load0 = [&](double2 (&v)[kRegs], i64 base) {
+        if constexpr (MIR) {
+            const double2* const lo = A.sv + base + tid;
+            const double2* const hi = A.sv + mtop - base - tid;
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[r] = __ldcs(lo + (r << 8));
+#pragma unroll
+            for (int r = 0; r < 8; r++) v[8 + r] = __ldcs(hi - (r << 8));
+        } else {
+#pragma unroll
+            for (int r = 0; r < kRegs; r++) v[r] = __ldcs(A.sv + base + thr_off + off0(r));
+        }
+    };
+    auto load1 = [&](double2 (&v)[kRegs], i64 base) {
+        if constexpr (MIR) {
+            const int t = lay_index<1>(tid, 0);
+            if (t < kTile / 2) {
+                const double2* const lo = A.sv + base + t;
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) v[r] = __ldcs(lo + (r << 4));
+            } else {
+                const double2* const hi = A.sv + mtop - base - (t - kTile / 2);
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) v[r] = __ldcs(hi - (r << 4));
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < kRegs; r++) v[r] = __ldcs(A.sv + base + thr_off1 + off1(r));
+        }
+    };
+    auto store0 = [&](const double2 (&v)[kRegs], i64 base) {
+        if constexpr (MIR) {
+            double2* const lo = A.sv + base + tid;
+            double2* const hi = A.sv + mtop - base - tid;
+#pragma unroll
+            for (int r = 0; r < 8; r++) __stcs(lo + (r << 8), v[r]);
+#pragma unroll
+            for (int r = 0; r < 8; r++) __stcs(hi - (r << 8), v[8 + r]);
+            if constexpr (ST == 2) {
+#pragma unroll
+                for (int r = 0; r < 8; r++) __stcs(A.sv + mfull - base - tid - (r << 8), v[r]);
+#pragma unroll
+                for (int r = 0; r < 8; r++)
+                    __stcs(A.sv + mtop + 1 + base + tid + (r << 8), v[8 + r]);
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < kRegs; r++) __stcs(A.sv + base + thr_off + off0(r), v[r]);
+            if constexpr (ST == 2) {
+#pragma unroll
+                for (int r = 0; r < kRegs; r++)
+                    __stcs(A.sv + mfull - base - thr_off - off0(r), v[r]);
+            }
+        }
+    };
+    auto store1 = [&](const double2 (&v)[kRegs], i64 base) {
+        if constexpr (MIR) {
+            const int t = lay_index<1>(tid, 0);
+            if (t < kTile / 2) {
+                double2* const lo = A.sv + base + t;
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) __stcs(lo + (r << 4), v[r]);
+                if constexpr (ST == 2) {
+                    double2* const up = A.sv + mfull - base - t;
+#pragma unroll
+                    for (int r = 0; r < kRegs; r++) __stcs(up - (r << 4), v[r]);
+                }
+            } else {
+                const i64 x = base + (t - kTile / 2);
+                double2* const hi = A.sv + mtop - x;
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) __stcs(hi - (r << 4), v[r]);
+                if constexpr (ST == 2) {
+                    double2* const up = A.sv + mtop + 1 + x;
+#pragma unroll
+                    for (int r = 0; r < kRegs; r++) __stcs(up + (r << 4), v[r]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < kRegs; r++) __stcs(A.sv + base + thr_off1 + off1(r), v[r]);
+            if constexpr (ST == 2) {
+#pragma unroll
+                for (int r = 0; r < kRegs; r++)
+                    __stcs(A.sv + mfull - base - thr_off1 - off1(r), v[r]);
+            }
+        }
+    };
 
     int par = 0;
     const i64 nunits = PAIR ? A.ntiles / 2 : A.ntiles;
@@ -796,7 +914,6 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
     for (i64 U = blockIdx.x; U < nunits; U += gridDim.x, par ^= 1) {
         const i64 T = PAIR ? 2 * U + grp : U;
         const i64 base = ((T & ((1ll << nmid) - 1)) << l) | ((T >> nmid) << (a + kTileBits - l));
-        double2* const p = A.sv + base + thr_off;
         double2 v[kRegs];
         // The loads go out first; the tile's cut constants are computed
         // while they are in flight.
@@ -806,14 +923,16 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
 #pragma unroll
             for (int r = 0; r < kRegs; r++) v[r] = own[pslot(lay_index<0>(0, r))];
         } else {
+            if (ALTM && par) {
+                load1(v, base);
+            } else if (LOAD) {
+                load0(v, base);
+            } else {
 #pragma unroll
-            for (int r = 0; r < kRegs; r++) {
-                if (ALTM && par) v[r] = __ldcs(A.sv + base + thr_off1 + off1(r));
-                else if (LOAD) v[r] = __ldcs(p + off0(r));
-                else v[r] = make_double2(0.0, 0.0);
+                for (int r = 0; r < kRegs; r++) v[r] = make_double2(0.0, 0.0);
             }
         }
-        if (!PAIR && LOAD && A.pf_dist > 0 && contiguous) {
+        if (!PAIR && LOAD && A.pf_dist > 0 && (contiguous || MIR)) {
             // Stream this CTA's tile pf_dist strides ahead from HBM into L2
             // (one bulk prefetch).  Strided tiles are not prefetched: per-
             // thread row prefetches cost more than they saved (12.2 against
@@ -821,11 +940,13 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
             // prefetch of the tile as a TMA box (61.5 against 58.1-61.0
             // layers/s at N=30, p=5; A/B in one call).
             const i64 T2 = T + (i64)A.pf_dist * gridDim.x;
-            if (T2 < A.ntiles && tid == 0) {
-                const i64 b2 = ((T2 & ((1ll << nmid) - 1)) << l) |
-                               ((T2 >> nmid) << (a + kTileBits - l));
+            if (T2 < A.ntiles && tid < (MIR ? 2 : 1)) {
+                i64 b2 = ((T2 & ((1ll << nmid) - 1)) << l) |
+                         ((T2 >> nmid) << (a + kTileBits - l));
+                constexpr int run = MIR ? kTile / 2 : kTile;  // a mirror tile is two runs
+                if (MIR && tid) b2 = mtop + 1 - run - b2;
                 asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.sv + b2),
-                             "r"((unsigned)(kTile * sizeof(double2)))
+                             "r"((unsigned)(run * sizeof(double2)))
                              : "memory");
             }
         }
@@ -921,8 +1042,7 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
             else
                 exchange<1, 0, PAIR>(v, buf, tid, false, grp);
             rx_regs<GM>(v, m_hi, A.gx, A.c, A.s);
-#pragma unroll
-            for (int r = 0; r < kRegs; r++) __stcs(p + off0(r), v[r]);
+            store0(v, base);
             continue;
         }
         if (ALTM && par) {  // the odd iteration of an alternating mixer pass (see ALTM)
@@ -931,8 +1051,7 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
             rx_regs<GM>(v, m_lo, A.gx, A.c, A.s);
             exchange<2, 0, PAIR>(v, buf, tid, false, grp);
             rx_regs<GM>(v, m_hi, A.gx, A.c, A.s);
-#pragma unroll
-            for (int r = 0; r < kRegs; r++) __stcs(p + off0(r), v[r]);
+            store0(v, base);
             continue;
         }
         if constexpr (PH == PH_MUL && !FUSED) {
@@ -980,14 +1099,17 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
                             const i64 T2 = PAIR ? 2 * U2 + grp : U2;
                             const i64 b2 = ((T2 & ((1ll << nmid) - 1)) << l) |
                                            ((T2 >> nmid) << (a + kTileBits - l));
-                            const double2* const src = A.sv + b2 + thr_off;
+                            const double2* const src = A.sv + b2 + (MIR ? tid : thr_off);
+                            const double2* const srch = A.sv + mtop - b2 - tid;
                             const unsigned dst = (unsigned)__cvta_generic_to_shared(
                                 buf + pbase<0>(tid));
 #pragma unroll
                             for (int r = 0; r < kRegs; r++)
                                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                                                  dst + (unsigned)(16 * pslot(lay_index<0>(0, r)))),
-                                             "l"(src + off0(r))
+                                             "l"(!MIR    ? src + off0(r)
+                                                 : r < 8 ? src + (r << 8)
+                                                         : srch - ((r & 7) << 8))
                                              : "memory");
                             asm volatile("cp.async.commit_group;" ::: "memory");
                         }
@@ -1028,14 +1150,10 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
             acc = t2;
         }
         if (ST) {
-            if (LAY == 0) {
-#pragma unroll
-                for (int r = 0; r < kRegs; r++) __stcs(p + off0(r), v[r]);
-            } else {
-                double2* const p1 = A.sv + base + thr_off1;
-#pragma unroll
-                for (int r = 0; r < kRegs; r++) __stcs(p1 + off1(r), v[r]);
-            }
+            if (LAY == 0)
+                store0(v, base);
+            else
+                store1(v, base);
         }
     }
     if (ACC) {

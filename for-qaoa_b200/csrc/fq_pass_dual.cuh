@@ -145,7 +145,12 @@ __host__ __device__ inline size_t dual_smem_bytes(int) {
 // Only psi is read (the state before the last forward pass); both vectors
 // are written as the reverse sweep's first pass would write them: 32 B
 // per amplitude instead of 32 + 48 + 64.
-template <typename WT, bool PHI, int SC, bool ST, int GM, int GM2 = GM_NONE, bool TURN = false>
+//
+// MIR: the mirror pass of a half state (see fq_pass.cuh); the gradient of a
+// circuit from |+>^N keeps both vectors as halves, and every sum here is
+// half of the whole state's (grad_collect doubles them).
+template <typename WT, bool PHI, int SC, bool ST, int GM, int GM2 = GM_NONE, bool TURN = false,
+          bool MIR = false>
 __global__ void __launch_bounds__(kPassThreads, 1)
     k_pass_dual(const PassArgs A, double* gb, double* gg, double* gb2) {
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -162,6 +167,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     constexpr bool CUT = PHI || TURN;
     constexpr bool INTW = sizeof(WT) == sizeof(int);
     constexpr bool FUSED = !TURN && GM2 != GM_NONE;
+    static_assert(!MIR || SC == SC_L021, "a mirror pass rotates tile bits 0..11");
     static_assert(PHI || !FUSED, "a fused adjoint pass carries its layer's phase");
     static_assert(!(PHI && TURN), "the turnaround pass carries no phase");
     constexpr int LP = SC == SC_L0 ? 0 : 1;  // layout after the first rounds
@@ -187,6 +193,8 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         return ((T & ((1ll << nmid) - 1)) << l) | ((T >> nmid) << (a + kTileBits - l));
     };
     const bool contiguous = (l == kTileBits);
+    // Element (b, t) of a mirror tile, b = tile bit 11: base + t or mtop - base - t.
+    const i64 mtop = (1ll << (N - 1)) - 1;
     const int pf_step = l < 3 ? l : 3;
     const unsigned m_hi = (A.tmask >> 8) & 15u, m_mid = (A.tmask >> 4) & 15u, m_lo = A.tmask & 15u;
     const int lo_lane = (SC != SC_L021 && m_lo) ? __ffs(m_lo) - 1 : -1;
@@ -213,17 +221,34 @@ __global__ void __launch_bounds__(kPassThreads, 1)
                 w[r] = own[kXTile + pslot(lay_index<0>(0, r))];
             }
         } else {
-            const i64 o = opaque(base + thr_off);
-            const i64 b8 = opaque(s8), b9 = opaque(s9), b10 = opaque(s10), b11 = opaque(s11);
+            if constexpr (MIR) {
+                const i64 o = opaque(base + tid), oh = opaque(mtop - base - tid);
 #pragma unroll
-            for (int r = 0; r < kRegs; r++) {
-                v[r] = __ldcs(A.sv + o + offr(r, b8, b9, b10, b11));
-                if (!TURN) w[r] = __ldcs(A.sv2 + o + offr(r, b8, b9, b10, b11));
+                for (int r = 0; r < kRegs; r++) {
+                    const i64 x = r < 8 ? o + (r << 8) : oh - ((r & 7) << 8);
+                    v[r] = __ldcs(A.sv + x);
+                    if (!TURN) w[r] = __ldcs(A.sv2 + x);
+                }
+            } else {
+                const i64 o = opaque(base + thr_off);
+                const i64 b8 = opaque(s8), b9 = opaque(s9), b10 = opaque(s10), b11 = opaque(s11);
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) {
+                    v[r] = __ldcs(A.sv + o + offr(r, b8, b9, b10, b11));
+                    if (!TURN) w[r] = __ldcs(A.sv2 + o + offr(r, b8, b9, b10, b11));
+                }
             }
         }
         if (T + gridDim.x < A.ntiles) {
             const i64 b2 = tile_base(T + gridDim.x);
-            if (contiguous) {
+            if (MIR) {  // two runs of each vector
+                if (tid < (TURN ? 2 : 4))
+                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
+                                     ((tid & 2) ? A.sv2 : A.sv) +
+                                     ((tid & 1) ? mtop + 1 - kTile / 2 - b2 : b2)),
+                                 "r"((unsigned)(kTile / 2 * sizeof(double2)))
+                                 : "memory");
+            } else if (contiguous) {
                 if (tid < (TURN ? 1 : 2))
                     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
                                      (tid ? A.sv2 : A.sv) + b2),
@@ -394,7 +419,9 @@ __global__ void __launch_bounds__(kPassThreads, 1)
                     // of both vectors there now.
                     have_next = T + gridDim.x < A.ntiles;
                     if (have_next) {
-                        const i64 o = opaque(tile_base(T + gridDim.x) + thr_off);
+                        const i64 b2 = tile_base(T + gridDim.x);
+                        const i64 o = opaque(b2 + (MIR ? tid : thr_off));
+                        const i64 oh = MIR ? opaque(mtop - b2 - tid) : 0;
                         const i64 b8 = opaque(s8), b9 = opaque(s9), b10 = opaque(s10),
                                   b11 = opaque(s11);
                         const unsigned dst =
@@ -402,7 +429,9 @@ __global__ void __launch_bounds__(kPassThreads, 1)
 #pragma unroll
                         for (int r = 0; r < kRegs; r++) {
                             const unsigned d = dst + (unsigned)(16 * pslot(lay_index<0>(0, r)));
-                            const i64 off = o + offr(r, b8, b9, b10, b11);
+                            const i64 off = !MIR    ? o + offr(r, b8, b9, b10, b11)
+                                            : r < 8 ? o + (r << 8)
+                                                    : oh - ((r & 7) << 8);
                             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d),
                                          "l"(A.sv + off)
                                          : "memory");
@@ -418,7 +447,31 @@ __global__ void __launch_bounds__(kPassThreads, 1)
             }
         }
         }  // !TURN
-        if (ST) {
+        if (ST && MIR) {
+            if (LAY == 0) {
+                const i64 o = opaque(base + tid), oh = opaque(mtop - base - tid);
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) {
+                    const i64 x = r < 8 ? o + (r << 8) : oh - ((r & 7) << 8);
+                    __stcs(A.sv + x, v[r]);
+                    __stcs(A.sv2 + x, w[r]);
+                }
+            } else if (lay_index<1>(tid, 0) < kTile / 2) {  // uniform across a warp
+                const i64 o = opaque(base + lay_index<1>(tid, 0));
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) {
+                    __stcs(A.sv + o + (r << 4), v[r]);
+                    __stcs(A.sv2 + o + (r << 4), w[r]);
+                }
+            } else {
+                const i64 o = opaque(mtop - base - (lay_index<1>(tid, 0) - kTile / 2));
+#pragma unroll
+                for (int r = 0; r < kRegs; r++) {
+                    __stcs(A.sv + o - (r << 4), v[r]);
+                    __stcs(A.sv2 + o - (r << 4), w[r]);
+                }
+            }
+        } else if (ST) {
             if (LAY == 0) {
                 const i64 o = opaque(base + thr_off);
                 const i64 b8 = opaque(s8), b9 = opaque(s9), b10 = opaque(s10), b11 = opaque(s11);

@@ -125,7 +125,7 @@ static_assert(tma_pass_smem_bytes<int>() <= 227 * 1024, "ring + tables fit one S
 static_assert(tma_pass_smem_bytes<double>() <= 227 * 1024, "ring + tables fit one SM (FP64)");
 static_assert(kMaxQubits * kMaxQubits * sizeof(double) <= kTileBytes, "weights fit one stage");
 
-template <typename WT, int PH, int GM, int EX, int SC>
+template <typename WT, int PH, int GM, int EX, int ST, int SC>
 __global__ void __launch_bounds__(kPassThreads, 1)
     k_pass_tma(const PassArgs A, const __grid_constant__ CUtensorMap tmap, const TmaGeom G) {
     extern __shared__ unsigned char smraw[];
@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     }
     const unsigned m_hi = (A.tmask >> 8) & 15u, m_mid = (A.tmask >> 4) & 15u, m_lo = A.tmask & 15u;
     const int lo_lane = (SC != SC_L021 && m_lo) ? __ffs(m_lo) - 1 : -1;
+    const i64 mfull = (1ll << N) - 1;  // ST = 2: the other half's index is mfull - x
     WT* const kp = ct.ke;  // written after a tile's first barrier, read after its second
     double acc = 0, comp = 0;
     i64 j = 0;
@@ -295,11 +296,17 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         if (LAY == 0) {
             double2* const p = A.sv + base + thr_off;
 #pragma unroll
-            for (int r = 0; r < kRegs; r++) __stcs(p + offtab[r], v[r]);
+            for (int r = 0; r < kRegs; r++) {
+                __stcs(p + offtab[r], v[r]);
+                if (ST == 2) __stcs(A.sv + mfull - base - thr_off - offtab[r], v[r]);
+            }
         } else {
             double2* const p1 = A.sv + base + thr_off1;
 #pragma unroll
-            for (int r = 0; r < kRegs; r++) __stcs(p1 + offtab[kRegs + r], v[r]);
+            for (int r = 0; r < kRegs; r++) {
+                __stcs(p1 + offtab[kRegs + r], v[r]);
+                if (ST == 2) __stcs(A.sv + mfull - base - thr_off1 - offtab[kRegs + r], v[r]);
+            }
         }
     }
     if (*s_abort) {

@@ -1,0 +1,61 @@
+"""GPU parity of whole circuits and gradients on half states (N >= 13: only
+the amplitudes with qubit N-1 = 0 are swept, the last pass writes both
+halves) at the edges of their tile geometries: one and two tiles (N=13, 14),
+rows of 16 and 8 amplitudes (N=20, 21), paired rows of 4 (N=22), the first
+size with three passes per layer (N=23), and the mirror pass as the last
+pass (even and odd P at two passes per layer)."""
+import numpy as np
+import pytest
+
+from conftest import (ENERGY_RTOL, GRAD_TOL, angles, assert_state_close, complete_int, gnp_fp,
+                      gnp_int)
+
+pytestmark = pytest.mark.gpu
+
+WIDE = 300000  # |w| up to this: integer weights beyond every phase table
+
+
+def graph(kind, n, rng):
+    if kind == "fp":
+        return gnp_fp(n, rng)
+    if kind == "wide":
+        return gnp_int(n, rng, lo=-WIDE, hi=WIDE)
+    return complete_int(n, rng, -7, 9)
+
+
+@pytest.mark.parametrize("n,P,kind", [(13, 1, "int"), (13, 2, "fp"), (14, 1, "fp"),
+                                      (14, 2, "wide"), (15, 3, "int"), (20, 1, "fp"),
+                                      (21, 2, "int"), (22, 1, "int"), (22, 2, "fp"),
+                                      (23, 1, "fp"), (23, 2, "int")])
+def test_half_state_forward(ctx, oracle, n, P, kind):
+    rng = np.random.default_rng(1000 * n + P)
+    W = graph(kind, n, rng)
+    g, b = angles(rng, P)
+    if kind == "wide":
+        g /= WIDE  # keep gamma * W at ordinary size
+    st = ctx.state(n)
+    try:
+        e = ctx.qaoa_forward(st, W, g, b)
+        psi = st.to_host()
+    finally:
+        st.free()
+    want = oracle.qaoa_logical(W, g, b)
+    assert_state_close(psi, want, what=f"N={n} P={P} {kind}")
+    eo = oracle.expectation(want, W)
+    assert abs(e - eo) <= ENERGY_RTOL * max(1.0, abs(eo), np.abs(W).sum())
+
+
+@pytest.mark.parametrize("n,P,kind", [(16, 1, "fp"), (16, 2, "int"), (17, 3, "wide"),
+                                      (20, 1, "int"), (21, 2, "fp")])
+def test_half_state_gradient(ctx, oracle, n, P, kind):
+    rng = np.random.default_rng(2000 * n + P)
+    W = graph(kind, n, rng)
+    g, b = angles(rng, P)
+    if kind == "wide":
+        g /= WIDE
+    e, gg, gb = ctx.energy_grad(n, W, g, b)
+    eo, go, bo = oracle.energy_grad(W, g, b)
+    scale = max(1.0, np.abs(go).max(), np.abs(bo).max())
+    assert abs(e - eo) <= ENERGY_RTOL * max(1.0, abs(eo), np.abs(W).sum())
+    assert np.abs(gg - go).max() <= GRAD_TOL * scale
+    assert np.abs(gb - bo).max() <= GRAD_TOL * scale
