@@ -207,11 +207,14 @@ int fq_ctx_create(int device, void* stream, fq_ctx** out) {
             cudaMalloc(&c->d_partial, sizeof(double) * c->partial_cap) != cudaSuccess ||
             cudaMalloc(&c->d_result, sizeof(double) * kResultWords) != cudaSuccess ||
             cudaMalloc(&c->d_scratch, kScratchBytes) != cudaSuccess ||
+            cudaMalloc(&c->d_tcut, kTcutBytes) != cudaSuccess ||
+            cudaMalloc(&c->d_img, kMaxGeoms * kImgStride) != cudaSuccess ||
             cudaMalloc(&c->d_err, sizeof(int)) != cudaSuccess ||
             cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess) {
             st = FQ_ERR_OOM;
             break;
         }
+        c->tcut_bytes = kTcutBytes;
         c->h_stage_bytes = std::max(wbytes, (size_t)256 * 1024);
         if (cudaMallocHost(&c->h_stage, c->h_stage_bytes) != cudaSuccess ||
             cudaMallocHost(&c->h_result, sizeof(double) * kResultWords) != cudaSuccess) {
@@ -244,6 +247,7 @@ int fq_ctx_destroy(fq_ctx* c) {
     cudaFree(c->d_err);
     cudaFree(c->d_scratch);
     cudaFree(c->d_tcut);
+    cudaFree(c->d_img);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->h_result) cudaFreeHost(c->h_result);
     if (c->stage_evt) cudaEventDestroy(c->stage_evt);

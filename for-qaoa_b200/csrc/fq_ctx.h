@@ -23,6 +23,7 @@ struct fq_ctx {
     size_t tcut_bytes = 0;
     long long tcut_version = -1;  // g_version the tables were built for (-1: none)
     int tcut_n = -1;              // and N
+    unsigned char* d_img = nullptr;  // static cut tables of the plan's geometries, built with them
     int partial_cap = 0;
     // Pinned host staging (uploads of weights and small tables).
     unsigned char* h_stage = nullptr;
@@ -53,6 +54,7 @@ namespace fq {
 
 constexpr int kResultWords = 4096;
 constexpr size_t kScratchBytes = 1 << 20;
+constexpr size_t kTcutBytes = 1 << 20;  // first size of d_tcut: circuits of up to 24 qubits
 
 // Host view of a graph, prepared for the kernels.
 struct GraphPrep {

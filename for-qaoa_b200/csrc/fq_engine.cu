@@ -45,17 +45,27 @@ __global__ void k_phase_table2(double2* tab, int dlo, int nhi, double gamma) {
 
 // Tables of k_phase_table2 for up to kMaxTableLayers layers in one launch:
 // layer p's table at tab + p * kTableStride.
+// The last block of x takes z^creg[r] of every geometry from the images at
+// img (WT per entry) instead; FP64 weights have nothing else (nhi = 0).
 struct LayerGammas {
     double g[kMaxTableLayers];
 };
 
-__global__ void k_phase_tables2(double2* tab, int dlo, int nhi, LayerGammas lg, int P) {
+template <typename WT>
+__global__ void k_phase_tables2(double2* tab, int dlo, int nhi, LayerGammas lg, int P,
+                                const unsigned char* img, int ngeom) {
     const int p = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
     double sn, cs;
     double2* t = tab + (size_t)p * kTableStride;
-    if (i < kPhaseLo) {
+    if (blockIdx.x == gridDim.x - 1) {
+        const int j = threadIdx.x;
+        if (j >= ngeom * kQtabStride) return;
+        const WT* creg = reinterpret_cast<const WT*>(img + (j / kQtabStride) * kImgStride);
+        sincos(lg.g[p] * (double)creg[j % kQtabStride], &sn, &cs);
+        t[kPhaseLo + kPhaseHiMax + j] = make_double2(cs, sn);
+    } else if (i < kPhaseLo) {
         sincos(lg.g[p] * (double)i, &sn, &cs);
         t[i] = make_double2(cs, sn);
     } else if (i < kPhaseLo + nhi) {
@@ -241,6 +251,7 @@ std::vector<PassPlan> plan_layer(int N, bool half) {
         std::swap(v[0], v[v.size() - 1]);
         std::swap(v[1], v[v.size() - 1]);
     }
+    for (size_t i = 0; i < v.size(); i++) v[i].geom = (int)i;
     return v;
 }
 
@@ -300,7 +311,13 @@ PassArgs engine_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g, const Pas
     A.a = p.a;
     A.tmask = p.tmask;
     A.mir = p.mir;
+    A.img = ctx->d_img + p.geom * kImgStride;
     return A;
+}
+
+void set_layer_tables(fq_ctx* ctx, PassArgs& A, const PassPlan& p, int layer) {
+    A.ptab = ctx->d_ptab + (size_t)layer * kTableStride;
+    A.qt = A.ptab + kPhaseLo + kPhaseHiMax + p.geom * kQtabStride;
 }
 
 // Range [dlo, dhi] of the powers of z the passes look up: every cut value
@@ -319,17 +336,22 @@ int engine_nhi(const GraphPrep& g) {
     return nhi <= kPhaseHiMax ? (int)nhi : 0;
 }
 
-int launch_tables2(fq_ctx* ctx, const GraphPrep& g, const double* gammas, int P) {
-    const int nhi = engine_nhi(g);
-    if (nhi == 0 || P > kMaxTableLayers) return FQ_ERR_INVALID;
+int launch_tables2(fq_ctx* ctx, const GraphPrep& g, const double* gammas, int P, int ngeom) {
+    const int nhi = g.integer ? engine_nhi(g) : 0;
+    if ((g.integer && nhi == 0) || P > kMaxTableLayers) return FQ_ERR_INVALID;
     long long dlo, dhi;
     table_range(g, dlo, dhi);
     LayerGammas lg;
     for (int p = 0; p < kMaxTableLayers; p++) lg.g[p] = p < P ? gammas[p] : 0.0;
-    const int n = kPhaseLo + nhi;
+    const int n = g.integer ? kPhaseLo + nhi : 0;
     const int tok = prof_begin(ctx);
-    k_phase_tables2<<<dim3((n + 255) / 256, P), 256, 0, ctx->stream>>>(ctx->d_ptab, (int)dlo, nhi,
-                                                                       lg, P);
+    const dim3 grid((n + 255) / 256 + 1, P);
+    if (g.integer)
+        k_phase_tables2<int><<<grid, 256, 0, ctx->stream>>>(ctx->d_ptab, (int)dlo, nhi, lg, P,
+                                                            ctx->d_img, ngeom);
+    else
+        k_phase_tables2<double><<<grid, 256, 0, ctx->stream>>>(ctx->d_ptab, 0, 0, lg, P,
+                                                               ctx->d_img, ngeom);
     FQ_CUDA(cudaGetLastError());
     prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
     ctx->launches++;
@@ -414,31 +436,32 @@ int setup_graph(fq_ctx* ctx, const double* graph, int N, GraphPrep& g) {
     return FQ_OK;
 }
 
-// Cut constants of every tile of each plan geometry (k_tile_cuts, one
-// launch) in ctx->d_tcut, grown on demand and kept while the weights and N
-// stay the same: tabs[i] serves plan[i].  Below
-// N = 21 (512 tiles) and without the buffer (a failed allocation) tabs
-// stays null and the passes compute the constants per tile, as they do for
-// shards and the read-only <C> pass.
-// The table is 64 B per tile (128 B with FP64 weights), 1/1024 of the
-// state per geometry; it replaces per-tile work on two warps of each tile
-// and the barrier after it.  On B200 at N=30, p=5, with the layer-0 pass
-// alternating its exchanges: layer-0 pass 5.26-5.32 against 5.66-5.78 ms,
-// fused passes 9.27-9.34 against 9.62-9.66, the circuit 79.1-79.6 against
-// 80.4-80.8 ms (A/B in one call).
+// The tables of a circuit's pass geometries that depend on the graph alone,
+// built by one launch (k_tile_cuts) and kept while the weights and N stay
+// the same: every tile's cut constants in ctx->d_tcut (grown on demand,
+// tabs[i] serves plan[i]; null when it cannot be had, the passes then
+// compute them per tile) and the static tables of each geometry in
+// ctx->d_img.  The tile constants are 64 B per tile (128 B with FP64
+// weights), 1/1024 of the swept state per geometry, and replace per-tile
+// work on two warps and the barrier after it.  The images replace each
+// CTA's own set-up from the weights, a chain of dependent shared-memory
+// reads and sincos before its first tile, which at one tile per CTA was half
+// of a pass.  On B200 (A/B in one call): forward N=20 p=5 112 against 140 us
+// with the set-up in every pass, N=23 p=4 (FP64 weights) 291 against 315 us;
+// gradient N=19 p=6 215 against 279 us; N >= 26 within 1%.
 static int tile_cut_tables(fq_ctx* ctx, const GraphPrep& g, int N,
                            const std::vector<PassPlan>& plan, std::vector<const void*>& tabs) {
     tabs.assign(plan.size(), nullptr);
-    if (N < 21 || plan.size() > 4) return FQ_OK;
+    FQ_CHECK(plan.size() <= kMaxGeoms, FQ_ERR_INVALID, "%zu passes per layer", plan.size());
     const size_t wt = g.integer ? sizeof(int) : sizeof(double);
-    const i64 ntiles = 1ll << (N - kTileBits - 1);  // a half state's
+    const i64 ntiles = 1ll << (N - kTileBits - (half_state(N) ? 1 : 0));
     const size_t per = (size_t)ntiles * kTcutStride * wt;
     const size_t need = per * plan.size();
     // Built for these weights (no upload since) and this N: reuse them, as
     // an optimiser's calls on one graph do.
-    if (ctx->d_tcut && need <= ctx->tcut_bytes && ctx->tcut_version == ctx->g_version &&
-        ctx->tcut_n == N) {
-        for (size_t i = 0; i < plan.size(); i++) tabs[i] = (char*)ctx->d_tcut + i * per;
+    if (ctx->tcut_version == ctx->g_version && ctx->tcut_n == N) {
+        for (size_t i = 0; i < plan.size() && need <= ctx->tcut_bytes; i++)
+            tabs[i] = (char*)ctx->d_tcut + i * per;
         return FQ_OK;
     }
     ctx->tcut_version = -1;
@@ -452,11 +475,14 @@ static int tile_cut_tables(fq_ctx* ctx, const GraphPrep& g, int N,
         if (cudaMalloc(&ctx->d_tcut, need) != cudaSuccess) {
             cudaGetLastError();  // clear the allocation failure
             ctx->d_tcut = nullptr;
-            return FQ_OK;
+        } else {
+            ctx->tcut_bytes = need;
         }
-        ctx->tcut_bytes = need;
     }
-    const int grid = (int)std::min<i64>((ntiles + 3) / 4, (i64)ctx->num_sms * 8);
+    const bool fits = need <= ctx->tcut_bytes;
+    const i64 nt = fits ? ntiles : 0;
+    // Eight blocks a SM at most; block 0 of each geometry also writes its image.
+    const int grid = (int)std::max<i64>(1, std::min<i64>((nt + 3) / 4, (i64)ctx->num_sms * 8));
     // The attribute is the same for every N: contexts on other threads (the
     // server's lanes) set it concurrently, and a launch needing more than
     // another thread's smaller setting would fail.
@@ -476,16 +502,16 @@ static int tile_cut_tables(fq_ctx* ctx, const GraphPrep& g, int N,
     }
     const dim3 grid2(grid, (unsigned)plan.size());
     if (g.integer)
-        k_tile_cuts<int><<<grid2, kPassThreads, smem, ctx->stream>>>((const int*)ctx->d_w, N, G,
-                                                                     ntiles, (int*)ctx->d_tcut);
+        k_tile_cuts<int><<<grid2, kPassThreads, smem, ctx->stream>>>(
+            (const int*)ctx->d_w, N, G, nt, (int*)ctx->d_tcut, ctx->d_img);
     else
         k_tile_cuts<double><<<grid2, kPassThreads, smem, ctx->stream>>>(
-            (const double*)ctx->d_w, N, G, ntiles, (double*)ctx->d_tcut);
+            (const double*)ctx->d_w, N, G, nt, (double*)ctx->d_tcut, ctx->d_img);
     FQ_CUDA(cudaGetLastError());
     ctx->launches++;
     ctx->tcut_version = ctx->g_version;
     ctx->tcut_n = N;
-    for (size_t i = 0; i < plan.size(); i++) tabs[i] = (char*)ctx->d_tcut + i * per;
+    for (size_t i = 0; i < plan.size() && fits; i++) tabs[i] = (char*)ctx->d_tcut + i * per;
     return FQ_OK;
 }
 
@@ -522,13 +548,12 @@ static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const Graph
         gate_params(betas[p], gm[p], gx[p], f);
         scale[p] = pow(f, N) * (p == 0 ? amp0 : 1.0);
     }
-    if (g.integer) FQ_TRY(launch_tables2(ctx, g, gammas, P));
-    // Phase arguments of layer q on a pass.
-    auto phase_args = [&](PassArgs& A, int q) {
-        if (g.integer) {
-            set_table_args(A, g, gammas[q], scale[q]);
-            A.ptab = ctx->d_ptab + (size_t)q * kTableStride;
-        }
+    const bool tables = P <= kMaxTableLayers;
+    if (tables) FQ_TRY(launch_tables2(ctx, g, gammas, P, npass));
+    // Phase arguments of layer q on a pass over plan[idx].
+    auto phase_args = [&](PassArgs& A, int q, int idx) {
+        if (g.integer) set_table_args(A, g, gammas[q], scale[q]);
+        if (tables) set_layer_tables(ctx, A, plan[idx], q);
         A.tree = phase_tree_ok(g, gammas[q]) ? 1 : 0;
         A.gamma = gammas[q];
         A.scale = g.integer ? 1.0 : scale[q];
@@ -543,11 +568,11 @@ static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const Graph
             const bool last_of_layer = j == npass - 1;
             int ph = PH_NONE;
             if (p == 0 && j == 0) {  // launch-control init + layer-0 phase + RX
-                phase_args(A, 0);
+                phase_args(A, 0, idx);
                 ph = PH_INIT;
                 FQ_TRY(dispatch_phase_pass(ctx, g.integer, PH_INIT, gm[0], A));
             } else if (last_of_layer && p + 1 < P) {
-                phase_args(A, p + 1);
+                phase_args(A, p + 1, idx);
                 A.gx2 = gx[p + 1];
                 ph = PH_MUL;
                 FQ_TRY(dispatch_fused(ctx, g.integer, gm[p], gm[p + 1], A));
@@ -595,11 +620,10 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
         // Two-level tables: all layers' in one launch (layer p's at slot p,
         // kept for the reverse sweep of a gradient); else one global table
         // per layer.
-        const bool all_tables = nhi > 0 && P <= kMaxTableLayers;
-        if (g.integer) {
-            if (all_tables) {
-                if (p == 0) FQ_TRY(launch_tables2(ctx, g, gammas, P));
-            } else if (nhi > 0) {
+        const bool all_tables = (nhi > 0 || !g.integer) && P <= kMaxTableLayers;
+        if (all_tables && p == 0) FQ_TRY(launch_tables2(ctx, g, gammas, P, (int)plan.size()));
+        if (g.integer && !all_tables) {
+            if (nhi > 0) {
                 FQ_TRY(launch_table2(ctx, g, gammas[p]));
             } else {
                 FQ_TRY(launch_table(ctx, g, gammas[p], scale));
@@ -612,7 +636,7 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
             A.tcut = tcut[i];
             A.gx = gx;
             if (nhi > 0) set_table_args(A, g, gammas[p], scale);
-            if (all_tables) A.ptab = ctx->d_ptab + (size_t)p * kTableStride;
+            if (all_tables) set_layer_tables(ctx, A, plan[i], p);
             A.tree = phase_tree_ok(g, gammas[p]) ? 1 : 0;
             A.gamma = gammas[p];
             A.scale = g.integer ? 1.0 : scale;

@@ -17,6 +17,7 @@ struct PassPlan {
     int l, a;
     unsigned tmask;
     int mir = 0;
+    int geom = 0;  // index in its plan: the place of its tables
 };
 
 // Passes of one layer for N >= 12: the contiguous tile over qubits 0..11
@@ -45,7 +46,11 @@ int engine_nhi(const GraphPrep& g);
 int launch_table2(fq_ctx* ctx, const GraphPrep& g, double gamma);
 // The same for layers 0..P-1 (P <= kMaxTableLayers) in one launch, layer p's
 // table at ctx->d_ptab + p * kTableStride.
-int launch_tables2(fq_ctx* ctx, const GraphPrep& g, const double* gammas, int P);
+// (FP64 weights: only z^creg[r] of the plan's ngeom geometries, which integer
+// weights get too; the images of tile_cut_tables come first).
+int launch_tables2(fq_ctx* ctx, const GraphPrep& g, const double* gammas, int P, int ngeom);
+// Points A at layer `layer`'s tables as launch_tables2 left them.
+void set_layer_tables(fq_ctx* ctx, PassArgs& A, const PassPlan& p, int layer);
 void set_table_args(PassArgs& A, const GraphPrep& g, double gamma, double scale);
 // FP64 weights: whether product-tree phases keep the phase arguments within
 // the reference's own rounding (|gamma| * sum|w| small).  Above the bound

@@ -235,7 +235,7 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     const int grid =
         (int)std::min<i64>(1ll << (N - kTileBits - (half ? 1 : 0)), (i64)ctx->num_sms);
     const bool batched = (i64)nrev * 3 * grid <= ctx->partial_cap && 3 * nrev <= kMaxGradSums;
-    const bool all_tables = g.integer && engine_nhi(g) > 0 && P <= kMaxTableLayers;
+    const bool all_tables = (!g.integer || engine_nhi(g) > 0) && P <= kMaxTableLayers;
     const int nhi = g.integer ? engine_nhi(g) : 0;
     std::vector<int> gm(P);
     std::vector<double> gx(P), f(P);
@@ -275,7 +275,7 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
             }
             A.gamma = gammas[k];
             if (nhi > 0) set_table_args(A, g, gammas[k], 1.0);
-            if (all_tables) A.ptab = ctx->d_ptab + (size_t)k * kTableStride;
+            if (all_tables) set_layer_tables(ctx, A, plan[i], k);
             A.tree = phase_tree_ok(g, gammas[k]) ? 1 : 0;
             // Inverse phase (times f^N) only where layers remain.
             A.scale = k > 0 ? pow(f[k], N) : 0.0;

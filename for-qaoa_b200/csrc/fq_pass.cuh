@@ -125,6 +125,12 @@ struct PassArgs {
     // tile (K, then e_0..e_11; k_tile_cuts), or null: each tile computes its
     // own (CutTables::tile, warps 0 and 1, then a barrier).
     const void* tcut;
+    // The geometry's static cut tables as k_tile_cuts wrote them (PassSmem
+    // from creg up to qtab), copied into shared memory instead of being
+    // rebuilt from the weights by every CTA; null: rebuilt.  qt: this layer's
+    // z^creg[r] of both layouts (k_phase_tables2), null: computed.
+    const void* img;
+    const double2* qt;
     int* err;        // device error flag (bounded waits that gave up)
     int mir;         // mirror pass of a half state (k_pass, k_pass_dual with MIR)
     int full;        // write both halves of the state (ST = 2)
@@ -136,7 +142,10 @@ constexpr int kPhaseLo = 32;     // low-part entries of the two-level phase tabl
 constexpr int kPhaseHiMax = 512; // high-part entries kept in shared memory at most
 // Layer tables of the two-level kind built in one launch, kTableStride
 // entries apart in the context's table buffer (kMaxPhaseTable entries).
-constexpr int kTableStride = kPhaseLo + kPhaseHiMax;
+constexpr int kMaxGeoms = 4;     // pass geometries of one engine plan at most
+constexpr int kQtabStride = 32;  // z^creg[r] of one geometry: 16 for L0, 16 for L1
+// A layer's slot: the two-level table, then the z^creg[r] of every geometry.
+constexpr int kTableStride = kPhaseLo + kPhaseHiMax + kMaxGeoms * kQtabStride;
 constexpr int kMaxTableLayers = 64;
 static_assert(kTableStride * kMaxTableLayers <= kMaxPhaseTable, "layer tables fit the buffer");
 
@@ -436,7 +445,35 @@ struct PassSmem {
     static constexpr size_t qtab = (thrc + 10 * kPassThreads * sizeof(WT) + 15) & ~(size_t)15;
     static constexpr size_t smtab = qtab + 32 * sizeof(double2);    // after 2 x 16 qtab
     static constexpr size_t bytes = smtab + sizeof(double2) * (kPhaseLo + kPhaseHiMax);
+    // Image of the static tables (creg, Dm, Ru, wf, wu, thrc).
+    static constexpr size_t img = qtab - creg;
+    static_assert(creg % 16 == 0 && img % 16 == 0, "the image is copied in 16-byte pieces");
 };
+constexpr size_t kImgStride = (PassSmem<double>::img + 255) & ~(size_t)255;
+
+// Starts the copy of a geometry's static tables, the layer's phase table
+// (tab, ntab entries) and its z^creg[r] (if any) into shared memory; the
+// caller waits (cp.async.wait_group 0 and a block barrier) before it reads
+// them.  Rebuilding them from the weights took every CTA several
+// microseconds of dependent shared-memory reads and a sincos before its
+// first tile (see tile_cut_tables, fq_engine.cu).
+template <typename WT>
+__device__ __forceinline__ void copy_tables(unsigned char* sm, const void* img,
+                                            const double2* tab, int ntab, const double2* qt) {
+    using SM = PassSmem<WT>;
+    auto cp = [](void* dst, const void* src) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         (unsigned)__cvta_generic_to_shared(dst)),
+                     "l"(src)
+                     : "memory");
+    };
+    for (int i = threadIdx.x; i < (int)(SM::img / 16); i += blockDim.x)
+        cp(sm + SM::creg + 16 * i, (const unsigned char*)img + 16 * i);
+    for (int i = threadIdx.x; i < ntab; i += blockDim.x) cp(sm + SM::smtab + 16 * i, tab + i);
+    if (qt && threadIdx.x < kQtabStride)
+        cp(sm + SM::qtab + 16 * threadIdx.x, qt + threadIdx.x);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
 
 // Shared-memory bytes k_pass needs (independent of N: the weights are
 // staged in the exchange buffer); a paired CTA has two exchange buffers.
@@ -535,11 +572,7 @@ struct CutTables {
                     if (((r >> k) ^ (r >> k2)) & 1)
                         c += sw[tile_phys(rbit(L, k), l, a) * N + tile_phys(rbit(L, k2), l, a)];
             creg[16 * L + r] = c;
-            if (QT) {
-                double sn, cs;
-                sincos(gamma * (double)c, &sn, &cs);
-                qtab[16 * L + r] = make_double2(cs, sn);
-            }
+            if (QT) qtab_entry(16 * L + r, gamma);
         }
         for (int L = 0; L < (THR ? 2 : 0); L++) {
             const int T = L == 0 ? tid : lay_index<1>(tid, 0);  // slot 0's tile index
@@ -566,6 +599,12 @@ struct CutTables {
             tc[tid] = athr;
             for (int k = 0; k < 4; k++) tc[(1 + k) * kPassThreads + tid] = f[k];
         }
+    }
+
+    __device__ void qtab_entry(int i, double gamma) const {
+        double sn, cs;
+        sincos(gamma * (double)creg[i], &sn, &cs);
+        qtab[i] = make_double2(cs, sn);
     }
 
     // Tile bit of register bit k and of thread bit j in layout L (L0: the
@@ -666,7 +705,8 @@ __host__ __device__ inline size_t tcut_smem_bytes(int N) {
 
 template <typename WT>
 __global__ void __launch_bounds__(kPassThreads) k_tile_cuts(const WT* w, int N, TcutGeoms G,
-                                                            i64 ntiles, WT* out) {
+                                                            i64 ntiles, WT* out,
+                                                            unsigned char* img) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int l = G.l[blockIdx.y], a = G.a[blockIdx.y];
     out += (i64)blockIdx.y * ntiles * kTcutStride;
@@ -674,8 +714,18 @@ __global__ void __launch_bounds__(kPassThreads) k_tile_cuts(const WT* w, int N, 
     const CutTables<WT> ct(smraw + ((N * N * sizeof(WT) + 15) & ~(size_t)15));
     for (int i = threadIdx.x; i < N * N; i += kPassThreads) sw[i] = w[i];
     __syncthreads();
-    ct.template setup<false, false>(sw, N, l, a, threadIdx.x, 0.0);
-    __syncthreads();
+    if (blockIdx.x == 0) {  // the geometry's image, once
+        using SM = PassSmem<WT>;
+        ct.template setup<false, true>(sw, N, l, a, threadIdx.x, 0.0);
+        __syncthreads();
+        const uint4* src = reinterpret_cast<const uint4*>(
+            smraw + ((N * N * sizeof(WT) + 15) & ~(size_t)15) + SM::creg);
+        uint4* dst = reinterpret_cast<uint4*>(img + blockIdx.y * kImgStride);
+        for (int i = threadIdx.x; i < (int)(SM::img / 16); i += kPassThreads) dst[i] = src[i];
+    } else {
+        ct.template setup<false, false>(sw, N, l, a, threadIdx.x, 0.0);
+        __syncthreads();
+    }
     const int nF = N - kTileBits, nmid = a - l, lane = threadIdx.x & 31;
     const int role = (threadIdx.x >> 5) & 1, tpb = kPassThreads / 64;  // tiles per block and round
     for (i64 T = (i64)blockIdx.x * tpb + (threadIdx.x >> 6); T < ntiles; T += (i64)gridDim.x * tpb) {
@@ -755,16 +805,22 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
 
     // ---- set-up: compact weight tables of this pass's tile geometry (the
     // tables depend on the geometry only: one copy serves both groups)
-    WT* sw = reinterpret_cast<WT*>(smraw);  // N*N weights while setting up
-    if (CUT) {
+    // The engine's passes copy the tables in while their first tile loads.
+    bool tables_pending = CUT && GM != GM_NONE && A.img;
+    if (tables_pending) {
+        copy_tables<WT>(sm, A.img, A.ptab,
+                        PH != PH_NONE && INTW && A.nhi > 0 ? kPhaseLo + A.nhi : 0,
+                        PH != PH_NONE ? A.qt : nullptr);
+    } else if (CUT) {
+        WT* sw = reinterpret_cast<WT*>(smraw);  // N*N weights while setting up
         const WT* gw = reinterpret_cast<const WT*>(A.w);
         for (int i = threadIdx.x; i < N * N; i += blockDim.x) sw[i] = gw[i];
+        if (PH != PH_NONE && INTW) load_phase_tables(A, smtab, threadIdx.x, blockDim.x);
+        __syncthreads();
+        if (threadIdx.x < kPassThreads)
+            ct.template setup<PH != PH_NONE>(sw, N, l, a, tid, A.gamma);
+        __syncthreads();  // the weights in the buffer are dead from here on
     }
-    if (PH != PH_NONE && INTW) load_phase_tables(A, smtab, threadIdx.x, blockDim.x);
-    __syncthreads();
-    if (CUT && threadIdx.x < kPassThreads)
-        ct.template setup<PH != PH_NONE>(sw, N, l, a, tid, A.gamma);
-    __syncthreads();  // the weights in the buffer are dead from here on
 
     // Address pieces: the thread's offsets in layouts L0 and L1 and the
     // strides of the 4 register bits of each (uniform across the grid).
@@ -953,6 +1009,15 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
         // The tile's cut constants: from the table (kp in global memory), or
         // computed by warps 0 and 1 into shared memory (double-buffered per
         // group: no barrier for the previous readers) and a barrier.
+        if (CUT && GM != GM_NONE && tables_pending) {
+            tables_pending = false;
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (PH != PH_NONE && !A.qt) {
+                if (threadIdx.x < kQtabStride) ct.qtab_entry(threadIdx.x, A.gamma);
+                __syncthreads();
+            }
+        }
         const WT* kp = ct.ke + 64 * grp + 32 * par;
         WT cbase = 0, g0 = 0, g1 = 0, g2 = 0, g3 = 0;
         if (CUT) {

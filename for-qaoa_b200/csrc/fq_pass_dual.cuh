@@ -173,15 +173,19 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     constexpr int LP = SC == SC_L0 ? 0 : 1;  // layout after the first rounds
     constexpr int LAY = (FUSED || TURN) ? 0 : LP;  // layout of the stores
 
-    WT* sw = reinterpret_cast<WT*>(buf);  // N*N weights while setting up
-    if (CUT) {
+    bool tables_pending = CUT && A.img;
+    if (tables_pending) {  // copied in while the first tile loads
+        copy_tables<WT>(sm, A.img, A.ptab, PHI && INTW && A.nhi > 0 ? kPhaseLo + A.nhi : 0,
+                        PHI ? A.qt : nullptr);
+    } else if (CUT) {
+        WT* sw = reinterpret_cast<WT*>(buf);  // N*N weights while setting up
         const WT* gw = reinterpret_cast<const WT*>(A.w);
         for (int i = tid; i < N * N; i += kPassThreads) sw[i] = gw[i];
         if (INTW) load_phase_tables(A, smtab, tid, kPassThreads);
+        __syncthreads();
+        ct.template setup<true>(sw, N, l, a, tid, A.gamma);
+        __syncthreads();  // the weights in buf are dead from here on
     }
-    __syncthreads();
-    if (CUT) ct.template setup<true>(sw, N, l, a, tid, A.gamma);
-    __syncthreads();  // the weights in buf are dead from here on
 
     const i64 thr_off = tile_off(tid, l, a);
     const i64 thr_off1 = tile_off(lay_index<1>(tid, 0), l, a);
@@ -260,6 +264,15 @@ __global__ void __launch_bounds__(kPassThreads, 1)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(A.sv + o) : "memory");
                     if (!TURN) asm volatile("prefetch.global.L2 [%0];" ::"l"(A.sv2 + o) : "memory");
                 }
+            }
+        }
+        if (CUT && tables_pending) {
+            tables_pending = false;
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (PHI && !A.qt) {
+                if (tid < kQtabStride) ct.qtab_entry(tid, A.gamma);
+                __syncthreads();
             }
         }
         WT* const kp = ct.ke + 32 * par;

@@ -182,8 +182,12 @@ __global__ void __launch_bounds__(kPassThreads, 1)
             if ((r >> k) & 1) o += 1ll << tile_phys(lo + k, l, a);
         offtab[tid] = o;
     }
+    // <C> with RX (a circuit's last pass): the cut tables come as an image.
+    constexpr bool IMG = PH == PH_NONE && CUT && GM != GM_NONE;
+    const bool img = IMG && A.img;
     WT* sw = reinterpret_cast<WT*>(stage + (size_t)(kStages - 1) * kTile);
-    if (CUT) {
+    if (img) copy_tables<WT>(tsm, A.img, nullptr, 0, nullptr);
+    if (CUT && !img) {
         const WT* gw = reinterpret_cast<const WT*>(A.w);
         for (int i = tid; i < N * N; i += kPassThreads) sw[i] = gw[i];
     }
@@ -191,7 +195,10 @@ __global__ void __launch_bounds__(kPassThreads, 1)
     __syncthreads();
     if (tid == 0)
         for (i64 j = 0; j < kStages - 1 && j < my_tiles; j++) issue(j);
-    if (CUT) ct.template setup<false>(sw, N, l, a, tid, A.gamma);
+    if (img)
+        asm volatile("cp.async.wait_group 0;" ::: "memory");  // read after the loop's barriers
+    else if (CUT)
+        ct.template setup<false>(sw, N, l, a, tid, A.gamma);
 
     i64 thr_off = 0, thr_off1 = 0;
     for (int jj = 0; jj < 8; jj++) thr_off |= (i64)((tid >> jj) & 1) << tile_phys(jj, l, a);

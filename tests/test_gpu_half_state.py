@@ -26,7 +26,9 @@ def graph(kind, n, rng):
 @pytest.mark.parametrize("n,P,kind", [(13, 1, "int"), (13, 2, "fp"), (14, 1, "fp"),
                                       (14, 2, "wide"), (15, 3, "int"), (20, 1, "fp"),
                                       (21, 2, "int"), (22, 1, "int"), (22, 2, "fp"),
-                                      (23, 1, "fp"), (23, 2, "int")])
+                                      (23, 1, "fp"), (23, 2, "int"),
+                                      # more layers than the shared layer tables hold
+                                      (14, 66, "fp"), (13, 65, "int")])
 def test_half_state_forward(ctx, oracle, n, P, kind):
     rng = np.random.default_rng(1000 * n + P)
     W = graph(kind, n, rng)
