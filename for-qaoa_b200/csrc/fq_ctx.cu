@@ -28,10 +28,9 @@ int validate_ctx(fq_ctx* ctx) {
 }
 
 int check_device_error(fq_ctx* ctx) {
-    int flag = 0;
-    FQ_CUDA(cudaMemcpy(&flag, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+    const int flag = *(volatile int*)ctx->err;
     if (flag) {
-        FQ_CUDA(cudaMemset(ctx->d_err, 0, sizeof(int)));
+        *(volatile int*)ctx->err = 0;
         set_error("a device-side bounded wait gave up (flag %d); results are incomplete", flag);
         return FQ_ERR_TIMEOUT;
     }
@@ -205,22 +204,20 @@ int fq_ctx_create(int device, void* stream, fq_ctx** out) {
         if (cudaMalloc(&c->d_w, wbytes) != cudaSuccess ||
             cudaMalloc(&c->d_ptab, sizeof(double2) * kMaxPhaseTable) != cudaSuccess ||
             cudaMalloc(&c->d_partial, sizeof(double) * c->partial_cap) != cudaSuccess ||
-            cudaMalloc(&c->d_result, sizeof(double) * kResultWords) != cudaSuccess ||
-            cudaMalloc(&c->d_scratch, kScratchBytes) != cudaSuccess ||
             cudaMalloc(&c->d_tcut, kTcutBytes) != cudaSuccess ||
-            cudaMalloc(&c->d_img, kMaxGeoms * kImgStride) != cudaSuccess ||
-            cudaMalloc(&c->d_err, sizeof(int)) != cudaSuccess ||
-            cudaMemset(c->d_err, 0, sizeof(int)) != cudaSuccess) {
+            cudaMalloc(&c->d_img, kMaxGeoms * kImgStride) != cudaSuccess) {
             st = FQ_ERR_OOM;
             break;
         }
         c->tcut_bytes = kTcutBytes;
         c->h_stage_bytes = std::max(wbytes, (size_t)256 * 1024);
         if (cudaMallocHost(&c->h_stage, c->h_stage_bytes) != cudaSuccess ||
-            cudaMallocHost(&c->h_result, sizeof(double) * kResultWords) != cudaSuccess) {
+            cudaMallocHost(&c->result, sizeof(double) * kResultWords + 64) != cudaSuccess) {
             st = FQ_ERR_OOM;
             break;
         }
+        c->err = (int*)(c->result + kResultWords);
+        *c->err = 0;
         if (cudaEventCreateWithFlags(&c->stage_evt, cudaEventDisableTiming) != cudaSuccess) {
             st = FQ_ERR_CUDA;
             break;
@@ -243,13 +240,10 @@ int fq_ctx_destroy(fq_ctx* c) {
     cudaFree(c->d_w);
     cudaFree(c->d_ptab);
     cudaFree(c->d_partial);
-    cudaFree(c->d_result);
-    cudaFree(c->d_err);
-    cudaFree(c->d_scratch);
     cudaFree(c->d_tcut);
     cudaFree(c->d_img);
     if (c->h_stage) cudaFreeHost(c->h_stage);
-    if (c->h_result) cudaFreeHost(c->h_result);
+    if (c->result) cudaFreeHost(c->result);
     if (c->stage_evt) cudaEventDestroy(c->stage_evt);
     for (auto& r : c->prof_pending) {
         cudaEventDestroy(r.a);

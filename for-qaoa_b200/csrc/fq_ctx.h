@@ -16,9 +16,13 @@ struct fq_ctx {
     void* d_w = nullptr;          // N*N weights (int32 or float64)
     double2* d_ptab = nullptr;    // integer phase table
     double* d_partial = nullptr;  // per-CTA reduction partials
-    double* d_result = nullptr;   // small device results (kResultWords)
-    unsigned char* d_scratch = nullptr;  // small-instance job data (kScratchBytes)
-    int* d_err = nullptr;         // kernels' error flag (nonzero: a bounded wait gave up)
+    // Results and the kernels' error flag (nonzero: a bounded wait gave up)
+    // live in pinned host memory that kernels write directly, so a call needs
+    // no copies behind its last kernel, only the stream's completion (on
+    // B200 the N=20 p=5 forward takes 88 us instead of 112, the N=19 p=6
+    // gradient 209 instead of 215, A/B in one call).
+    double* result = nullptr;     // kResultWords
+    int* err = nullptr;
     void* d_tcut = nullptr;       // per-tile cut constants of the engine's passes (grown on demand)
     size_t tcut_bytes = 0;
     long long tcut_version = -1;  // g_version the tables were built for (-1: none)
@@ -28,7 +32,6 @@ struct fq_ctx {
     // Pinned host staging (uploads of weights and small tables).
     unsigned char* h_stage = nullptr;
     size_t h_stage_bytes = 0;
-    double* h_result = nullptr;
     cudaEvent_t stage_evt = nullptr;
     // Graph cache: the last weights uploaded to d_w.
     std::vector<double> g_key;
@@ -53,7 +56,6 @@ struct fq_ctx {
 namespace fq {
 
 constexpr int kResultWords = 4096;
-constexpr size_t kScratchBytes = 1 << 20;
 constexpr size_t kTcutBytes = 1 << 20;  // first size of d_tcut: circuits of up to 24 qubits
 
 // Host view of a graph, prepared for the kernels.

@@ -31,7 +31,7 @@ __global__ void k_selftest_wait(int* err, long long max_polls) {
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     const bool done = mbar_wait_polls(&bar, 0, max_polls);
-    if (!done && threadIdx.x == 0) atomicExch(err, 2);
+    if (!done && threadIdx.x == 0) *(volatile int*)err = 2;
 }
 
 }  // namespace fq
@@ -39,7 +39,7 @@ __global__ void k_selftest_wait(int* err, long long max_polls) {
 extern "C" int fq_ctx_selftest_wait(fq_ctx* ctx) {
     using namespace fq;
     FQ_TRY(validate_ctx(ctx));
-    k_selftest_wait<<<1, 32, 0, ctx->stream>>>(ctx->d_err, 1ll << 16);
+    k_selftest_wait<<<1, 32, 0, ctx->stream>>>(ctx->err, 1ll << 16);
     FQ_CUDA(cudaGetLastError());
     ctx->launches++;
     return FQ_OK;

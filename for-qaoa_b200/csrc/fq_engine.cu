@@ -300,13 +300,13 @@ PassArgs base_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g) {
     A.W = g.integer ? (double)g.W_int : g.W;
     A.scale = 1.0;
     A.pf_dist = prefetch_distance();
-    A.err = ctx->d_err;
+    A.err = ctx->err;
     return A;
 }
 
 PassArgs engine_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g, const PassPlan& p) {
     PassArgs A = base_args(ctx, sv, N, g);
-    if (half_state(N)) A.ntiles >>= 1;
+    A.ntiles >>= 1;  // a half state's
     A.l = p.l;
     A.a = p.a;
     A.tmask = p.tmask;
@@ -397,11 +397,9 @@ int launch_table(fq_ctx* ctx, const GraphPrep& g, double gamma, double scale) {
 }
 
 int read_result(fq_ctx* ctx, double* host) {
-    FQ_CUDA(cudaMemcpyAsync(ctx->h_result, ctx->d_result, sizeof(double), cudaMemcpyDeviceToHost,
-                            ctx->stream));
     FQ_CUDA(cudaStreamSynchronize(ctx->stream));
     FQ_TRY(check_device_error(ctx));
-    *host = ctx->h_result[0];
+    *host = *(volatile double*)ctx->result;
     return FQ_OK;
 }
 
@@ -415,7 +413,7 @@ int reduce_partials(fq_ctx* ctx, const double* partial, int n, double* out_dev) 
 }
 
 int reduce_to_result(fq_ctx* ctx, int n) {
-    k_reduce_partials<<<1, 256, 0, ctx->stream>>>(ctx->d_partial, n, ctx->d_result);
+    k_reduce_partials<<<1, 256, 0, ctx->stream>>>(ctx->d_partial, n, ctx->result);
     FQ_CUDA(cudaGetLastError());
     ctx->launches++;
     return FQ_OK;
@@ -454,7 +452,7 @@ static int tile_cut_tables(fq_ctx* ctx, const GraphPrep& g, int N,
     tabs.assign(plan.size(), nullptr);
     FQ_CHECK(plan.size() <= kMaxGeoms, FQ_ERR_INVALID, "%zu passes per layer", plan.size());
     const size_t wt = g.integer ? sizeof(int) : sizeof(double);
-    const i64 ntiles = 1ll << (N - kTileBits - (half_state(N) ? 1 : 0));
+    const i64 ntiles = 1ll << (N - kTileBits - 1);  // a half state's
     const size_t per = (size_t)ntiles * kTcutStride * wt;
     const size_t need = per * plan.size();
     // Built for these weights (no upload since) and this N: reuse them, as
@@ -524,7 +522,7 @@ bool fuse_enabled() {
     return m != 0;
 }
 
-// The fused forward circuit for N >= 12 (see fq_qaoa_forward); with energy
+// The fused forward circuit (see fq_qaoa_forward); with energy
 // != NULL the last sweep also sums <C> and *energy receives it.
 
 // The fused schedule: layer p visits its passes in plan order when p is even
@@ -587,25 +585,24 @@ static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const Graph
     return FQ_OK;
 }
 
-bool engine_fused(const GraphPrep& g, int N, int P) {
-    return fuse_enabled() && half_state(N) && P >= 2 &&
+bool engine_fused(const GraphPrep& g, int P) {
+    return fuse_enabled() && P >= 2 &&
            (!g.integer || (engine_nhi(g) > 0 && P <= kMaxTableLayers));
 }
 
 int engine_last_pass(const GraphPrep& g, int N, int P) {
-    const int npass = (int)plan_layer(N, half_state(N)).size();
-    return (engine_fused(g, N, P) && (P - 1) % 2 == 1) ? 0 : npass - 1;
+    const int npass = (int)plan_layer(N, true).size();
+    return (engine_fused(g, P) && (P - 1) % 2 == 1) ? 0 : npass - 1;
 }
 
 int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, const double* gammas,
                    const double* betas, double* energy, bool skip_last) {
     const double amp0 = fq_init_amp(N);
-    const std::vector<PassPlan> plan = plan_layer(N, half_state(N));
+    const std::vector<PassPlan> plan = plan_layer(N, true);
     int last_grid = 0;
-    const bool fused = engine_fused(g, N, P);
-    FQ_CHECK(!(skip_last && (energy || plan.size() < 2)), FQ_ERR_INVALID,
-             "the forward circuit can stop before its last pass only without <C> and with two "
-             "or more passes per layer");
+    const bool fused = engine_fused(g, P);
+    FQ_CHECK(!(skip_last && energy), FQ_ERR_INVALID,
+             "the forward circuit can stop before its last pass only without <C>");
     std::vector<const void*> tcut;
     FQ_TRY(tile_cut_tables(ctx, g, N, plan, tcut));
     if (fused)
@@ -632,7 +629,7 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
         for (size_t i = 0; i < plan.size(); i++) {
             if (skip_last && p == P - 1 && i + 1 == plan.size()) break;
             PassArgs A = engine_args(ctx, sv, N, g, plan[i]);
-            A.full = half_state(N) && p == P - 1 && i + 1 == plan.size();
+            A.full = p == P - 1 && i + 1 == plan.size();
             A.tcut = tcut[i];
             A.gx = gx;
             if (nhi > 0) set_table_args(A, g, gammas[p], scale);
@@ -641,7 +638,7 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
             A.gamma = gammas[p];
             A.scale = g.integer ? 1.0 : scale;
             const int ph = i == 0 ? (p == 0 ? PH_INIT : PH_MUL) : PH_NONE;
-            const int ex = (energy && p == P - 1 && i + 1 == plan.size() && i > 0) ? 1 : 0;
+            const int ex = energy && A.full ? 1 : 0;
             if (ph != PH_NONE)
                 FQ_TRY(dispatch_phase_pass(ctx, g.integer, ph, gm, A));
             else
@@ -650,14 +647,9 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
         }
     }
     if (energy) {
-        if (plan.size() == 1) {  // the only pass carries the phase: <C> in its own sweep
-            PassArgs A = base_args(ctx, sv, N, g);
-            FQ_TRY(dispatch_readonly(ctx, g.integer, false, A));
-            last_grid = pass_grid(ctx, A, PH_NONE, false);
-        }
         FQ_TRY(reduce_to_result(ctx, last_grid));
         FQ_TRY(read_result(ctx, energy));
-        if (half_state(N)) *energy *= 2.0;  // the swept half's sum
+        *energy *= 2.0;  // the swept half's sum
     }
     return FQ_OK;
 }
@@ -678,29 +670,12 @@ int fq_qaoa_forward(fq_ctx* ctx, void* sv, int N, int P, const double* graph,
         FQ_CHECK(isfinite(gammas[p]) && isfinite(betas[p]), FQ_ERR_INVALID,
                  "non-finite angle at layer %d", p);
     GraphPrep g;
-    FQ_TRY(setup_graph(ctx, graph, N, g));
-    const double amp0 = fq_init_amp(N);
-    if (N < kTileBits) {
-        Targets T;
-        for (int q = 0; q < N; q++) T.t[q] = q;
-        for (int p = 0; p < P; p++) {
-            k_cost_small<<<1, 1024, 0, ctx->stream>>>((double2*)sv, N, gammas[p],
-                                                      (const double*)ctx->d_w, p == 0, amp0);
-            k_rx_small<<<1, 1024, 0, ctx->stream>>>((double2*)sv, N, T, N, cos(betas[p] / 2),
-                                                    sin(betas[p] / 2));
-            ctx->launches += 2;
-        }
-        FQ_CUDA(cudaGetLastError());
-        if (energy) {
-            k_cut_small<<<1, 256, 0, ctx->stream>>>((const double2*)sv, N,
-                                                    (const double*)ctx->d_w, ctx->d_result,
-                                                    nullptr);
-            FQ_CUDA(cudaGetLastError());
-            ctx->launches++;
-            FQ_TRY(read_result(ctx, energy));
-        }
-        return FQ_OK;
+    if (N <= kSmallKernelQubits) {
+        FQ_TRY(prep_graph(graph, N, g));
+        FQ_TRY(run_small(ctx, g, P, gammas, betas, SJ_STATE, (double2*)sv, ctx->result));
+        return energy ? read_result(ctx, energy) : FQ_OK;
     }
+    FQ_TRY(setup_graph(ctx, graph, N, g));
     return engine_forward(ctx, sv, N, P, g, gammas, betas, energy);
 }
 
@@ -712,7 +687,7 @@ int fq_expectation(fq_ctx* ctx, const void* sv, int N, const double* graph, doub
     FQ_TRY(setup_graph(ctx, graph, N, g));
     if (N < kTileBits) {
         k_cut_small<<<1, 256, 0, ctx->stream>>>((const double2*)sv, N, (const double*)ctx->d_w,
-                                                ctx->d_result, nullptr);
+                                                ctx->result, nullptr);
         FQ_CUDA(cudaGetLastError());
         ctx->launches++;
         return read_result(ctx, energy);

@@ -23,18 +23,15 @@ struct PassPlan {
 // Passes of one layer for N >= 12: the contiguous tile over qubits 0..11
 // and strided tiles over the remaining qubits (the first strided one leads
 // when there are three or more passes); the first pass carries the phase.
-// half (N >= 13): the passes of a half state, the mirror tile over qubits
-// 0..10 and N-1 and strided tiles over qubits 11..N-2.
+// half: the passes of a half state, the mirror tile over qubits 0..10 and
+// N-1 and strided tiles over qubits 11..N-2.
 std::vector<PassPlan> plan_layer(int N, bool half = false);
-// Whether whole circuits from |+>^N run on a half state (fq_pass.cuh): every
-// N whose half fills a tile.  The passes are bound by on-chip work and HBM
-// traffic per amplitude, and both halve.  On B200, against sweeping the
-// whole state (A/B in one call): forward N=30 p=5 40.0 against 77.6 ms, N=28
-// p=3 with FP64 weights 6.20 against 11.87 ms, N=23 p=4 0.315 against
-// 0.493 ms; gradient N=26 p=10 15.5 against 30.7 ms.  At N <= 20 the
-// passes' set-up and latency dominate: forward N=20 p=5 140 against 164 us.
-inline bool half_state(int N) { return N > kTileBits; }
-// Pass arguments of plan entry p on the engine's state (half for N >= 13).
+// Pass arguments of plan entry p on a whole circuit's half state
+// (fq_pass.cuh).  The passes are bound by on-chip work and HBM traffic per
+// amplitude, and both halve.  On B200, against sweeping the whole state (A/B
+// in one call): forward N=30 p=5 40.0 against 77.6 ms, N=28 p=3 with FP64
+// weights 6.20 against 11.87 ms, N=23 p=4 0.315 against 0.493 ms; gradient
+// N=26 p=10 15.5 against 30.7 ms.
 PassArgs engine_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g, const PassPlan& p);
 // Reduced RX for angle beta: gate mode, t or u, and the factor f.
 void gate_params(double beta, int& gm, double& g, double& f);
@@ -65,7 +62,7 @@ bool fuse_enabled();
 // Fixed-order sum of n partials into one device word.
 int reduce_partials(fq_ctx* ctx, const double* partial, int n, double* out_dev);
 int reduce_to_result(fq_ctx* ctx, int n);
-// Copies ctx->d_result[0] to *host (synchronises).
+// Waits for the stream and reads ctx->result[0].
 int read_result(fq_ctx* ctx, double* host);
 int check_state(void* sv, int N);
 // RX(angle) (full form) on every qubit whose bit is set in mask (fq_rx_targets).
@@ -77,10 +74,10 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
                    const double* betas, double* energy, bool skip_last = false);
 // Whether engine_forward uses the fused two-layer schedule, and the plan
 // index of the last pass it runs.
-bool engine_fused(const GraphPrep& g, int N, int P);
+bool engine_fused(const GraphPrep& g, int P);
 int engine_last_pass(const GraphPrep& g, int N, int P);
 
-// The N >= 13 gradient split for asynchronous use: grad_enqueue puts every
+// The gradient of more than kSmallJobMaxQubits qubits split for asynchronous use: grad_enqueue puts every
 // kernel and the final device-to-host copy of the results on ctx's stream;
 // once the stream has passed that point, grad_collect assembles them.
 int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const double* graph,
@@ -88,9 +85,17 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
 int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,
                  double* grad_beta);
 
-// k_small_jobs (fq_small.cuh) over jobs ordered by size class
-// (small_class): counts[c] jobs of class c, one launch per class present;
-// nmax0 = the largest N of class 0.
-int launch_small_jobs(const SmallJob* jobs, const int* counts, int nmax0, cudaStream_t stream);
+// Small instances (fq_small.cuh, N <= kSmallKernelQubits).  small_job fills a
+// descriptor (its pointers apart) and its small_words(N, P) data words: the
+// weights, then the layers.
+// alone: the job is launched by itself (run_small), not in a batch.
+void small_job(const GraphPrep& g, int P, const double* gammas, const double* betas, int flags,
+               bool alone, SmallJob& J, double* data);
+// Enqueues one instance on ctx's stream; out (1 + 2P words with SJ_GRAD,
+// else 1) and state (SJ_STATE) are device-accessible.
+int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
+              int flags, double2* state, double* out);
+// Gradients of njobs instances of size class c, descriptors on the device.
+int launch_small_batch(const SmallJob* jobs, int njobs, int c, cudaStream_t stream);
 
 }  // namespace fq

@@ -1,6 +1,6 @@
 // fq_grad.cu -- <C> and its adjoint gradient with respect to every gamma_k
-// and beta_k in one forward and one reverse sweep (fq_qaoa_energy_grad), and
-// batches of small instances in one launch (fq_small_batch).
+// and beta_k in one forward and one reverse sweep (fq_qaoa_energy_grad); up
+// to kSmallKernelQubits qubits on chip (fq_small.cuh).
 #include <math.h>
 #include <string.h>
 
@@ -11,7 +11,6 @@
 #include "fq_engine.h"
 #include "fq_launch.cuh"
 #include "fq_disp_dual.cuh"
-#include "fq_small.cuh"
 
 namespace fq {
 
@@ -47,126 +46,6 @@ __global__ void k_reduce_grad(const double* part, int grid, const GradSums S, do
     if (threadIdx.x == 0) out[d] = sh[0];
 }
 
-// n jobs of one size class: CB = 0 (N <= 12, one CTA each, nl = the
-// largest N) or CB = N - 12 (a cluster of 2^CB CTAs each, nl = 12).
-template <int CB>
-static int launch_small_class(const SmallJob* jobs, int n, int nl, cudaStream_t stream) {
-    auto fn = k_small_jobs<CB>;
-    FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)small_smem_bytes(kSmallMaxQubits)));
-    if (CB == 0) {
-        fn<<<n, kSmallThreads, small_smem_bytes(nl), stream>>>(jobs, n);
-        FQ_CUDA(cudaGetLastError());
-        return FQ_OK;
-    }
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)n << CB);
-    cfg.blockDim = dim3(kSmallThreads);
-    cfg.dynamicSmemBytes = small_smem_bytes(kSmallMaxQubits);
-    cfg.stream = stream;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 1u << CB;
-    at.val.clusterDim.y = 1;
-    at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    FQ_CUDA(cudaLaunchKernelEx(&cfg, fn, jobs, n));
-    return FQ_OK;
-}
-
-int launch_small_jobs(const SmallJob* jobs, const int* counts, int nmax0, cudaStream_t stream) {
-    int off = 0;
-    for (int c = 0; c <= kSmallJobMaxQubits - kSmallMaxQubits; c++) {
-        if (counts[c] == 0) continue;
-        switch (c) {
-            case 0: FQ_TRY(launch_small_class<0>(jobs, counts[0], nmax0, stream)); break;
-            case 1: FQ_TRY(launch_small_class<1>(jobs + off, counts[1], 12, stream)); break;
-            case 2: FQ_TRY(launch_small_class<2>(jobs + off, counts[2], 12, stream)); break;
-            default: FQ_TRY(launch_small_class<3>(jobs + off, counts[3], 12, stream)); break;
-        }
-        off += counts[c];
-    }
-    return FQ_OK;
-}
-
-// Upload a batch of small jobs (descriptors + their data) through the
-// pinned staging buffer into ctx->d_scratch and launch one CTA per job.
-// data: per job, N*N weights, P gammas, P betas (doubles, host); outputs go
-// to d_result starting at word out_base.
-struct SmallHostJob {
-    int N, P, flags;
-    const double* w;  // N*N symmetric (host)
-    const double* gammas;
-    const double* betas;
-    double2* state;   // device or null
-};
-
-static int run_small_jobs(fq_ctx* ctx, const SmallHostJob* jobs, int njobs, int out_base,
-                          std::vector<int>& out_off) {
-    size_t need = sizeof(SmallJob) * njobs;
-    int nmax = 1, outw = 0;
-    for (int i = 0; i < njobs; i++) {
-        need += sizeof(double) * (jobs[i].N * jobs[i].N + 2 * jobs[i].P);
-        if (small_class(jobs[i].N) == 0) nmax = std::max(nmax, jobs[i].N);  // class 0's largest
-        outw += 1 + 2 * jobs[i].P;
-    }
-    FQ_CHECK(need <= ctx->h_stage_bytes && need <= kScratchBytes, FQ_ERR_INVALID,
-             "small batch too large for the staging buffer (%zu bytes)", need);
-    FQ_CHECK(out_base + outw <= kResultWords, FQ_ERR_INVALID, "too many small-job outputs");
-    FQ_TRY(stage_acquire(ctx));
-    unsigned char* h = ctx->h_stage;
-    SmallJob* hj = reinterpret_cast<SmallJob*>(h);
-    double* hd = reinterpret_cast<double*>(h + sizeof(SmallJob) * njobs);
-    const double* dd = reinterpret_cast<const double*>(ctx->d_scratch + sizeof(SmallJob) * njobs);
-    size_t off = 0;
-    int o = out_base;
-    out_off.assign(njobs, 0);
-    for (int i = 0; i < njobs; i++) {
-        const SmallHostJob& J = jobs[i];
-        SmallJob d;
-        d.N = J.N;
-        d.P = J.P;
-        d.flags = J.flags;
-        d.pad = 0;
-        memcpy(hd + off, J.w, sizeof(double) * J.N * J.N);
-        d.w = dd + off;
-        off += J.N * J.N;
-        memcpy(hd + off, J.gammas, sizeof(double) * J.P);
-        d.gammas = dd + off;
-        off += J.P;
-        memcpy(hd + off, J.betas, sizeof(double) * J.P);
-        d.betas = dd + off;
-        off += J.P;
-        d.out = ctx->d_result + o;
-        out_off[i] = o;
-        o += 1 + 2 * J.P;
-        d.state = J.state;
-        hj[i] = d;
-    }
-    FQ_CUDA(cudaMemcpyAsync(ctx->d_scratch, h, need, cudaMemcpyHostToDevice, ctx->stream));
-    FQ_CUDA(cudaEventRecord(ctx->stage_evt, ctx->stream));
-    const int tok = prof_begin(ctx);
-    int counts[kSmallClasses] = {};
-    for (int i = 0; i < njobs; i++) counts[small_class(jobs[i].N)]++;
-    for (int i = 1; i < njobs; i++)
-        FQ_CHECK(small_class(jobs[i].N) >= small_class(jobs[i - 1].N), FQ_ERR_INVALID,
-                 "small jobs must come ordered by size class");
-    FQ_TRY(launch_small_jobs(reinterpret_cast<const SmallJob*>(ctx->d_scratch), counts, nmax,
-                             ctx->stream));
-    prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
-    ctx->launches++;
-    return FQ_OK;
-}
-
-static int read_results(fq_ctx* ctx, int words) {
-    FQ_CUDA(cudaMemcpyAsync(ctx->h_result, ctx->d_result, sizeof(double) * words,
-                            cudaMemcpyDeviceToHost, ctx->stream));
-    FQ_CUDA(cudaStreamSynchronize(ctx->stream));
-    return check_device_error(ctx);
-}
-
 static int check_angles(int P, const double* gammas, const double* betas) {
     FQ_CHECK(P >= 1 && gammas && betas, FQ_ERR_INVALID, "need P >= 1 and angle arrays");
     for (int p = 0; p < P; p++)
@@ -175,8 +54,8 @@ static int check_angles(int P, const double* gammas, const double* betas) {
     return FQ_OK;
 }
 
-// Enqueue the gradient of an N >= 13 circuit on ctx's stream; the results
-// land in ctx->h_result once the stream reaches this point (grad_collect).
+// Enqueue the gradient of a circuit with buffers on ctx's stream; the results
+// land in ctx->result once the stream reaches this point (grad_collect).
 int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const double* graph,
                  const double* gammas, const double* betas) {
     FQ_TRY(check_angles(P, gammas, betas));
@@ -184,11 +63,14 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     FQ_TRY(check_state(costate, N));
     FQ_CHECK(sv != costate, FQ_ERR_INVALID, "state and costate must be different buffers");
     GraphPrep g;
-    FQ_TRY(setup_graph(ctx, graph, N, g));
-    const bool half = half_state(N);
-    const std::vector<PassPlan> plan = plan_layer(N, half);
+    const std::vector<PassPlan> plan = plan_layer(N, true);
     const int npass = (int)plan.size();
     FQ_CHECK(1 + P + P * npass < kResultWords, FQ_ERR_INVALID, "P=%d too large", P);
+    if (N <= kSmallKernelQubits) {
+        FQ_TRY(prep_graph(graph, N, g));
+        return run_small(ctx, g, P, gammas, betas, SJ_GRAD, nullptr, ctx->result);
+    }
+    FQ_TRY(setup_graph(ctx, graph, N, g));
 
     // Reverse sweep.  Layer k visits its passes in the reverse of the
     // forward order (descending plan order for even k, ascending for odd
@@ -226,14 +108,13 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     FQ_TRY(engine_forward(ctx, sv, N, P, g, gammas, betas, nullptr, turn));
     if (!turn) {
         PassArgs A = base_args(ctx, sv, N, g);
-        if (half) A.ntiles >>= 1;
+        A.ntiles >>= 1;  // the half state
         A.sv2 = (double2*)costate;
         FQ_TRY(dispatch_costate(ctx, g.integer, A));
         FQ_TRY(reduce_partials(ctx, ctx->d_partial, pass_grid(ctx, A, PH_NONE, false),
-                               ctx->d_result));
+                               ctx->result));
     }
-    const int grid =
-        (int)std::min<i64>(1ll << (N - kTileBits - (half ? 1 : 0)), (i64)ctx->num_sms);
+    const int grid = (int)std::min<i64>(1ll << (N - kTileBits - 1), (i64)ctx->num_sms);
     const bool batched = (i64)nrev * 3 * grid <= ctx->partial_cap && 3 * nrev <= kMaxGradSums;
     const bool all_tables = (!g.integer || engine_nhi(g) > 0) && P <= kMaxTableLayers;
     const int nhi = g.integer ? engine_nhi(g) : 0;
@@ -300,40 +181,34 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
             if (energy_here) sums.dst[3 * q + 1] = 0;
             if (R.fused) sums.dst[3 * q + 2] = dst_b2;
         } else {
-            FQ_TRY(reduce_partials(ctx, gb, grid, ctx->d_result + dst_b));
-            if (energy_here) FQ_TRY(reduce_partials(ctx, gg, grid, ctx->d_result));
-            if (R.phi) FQ_TRY(reduce_partials(ctx, gg, grid, ctx->d_result + dst_g));
-            if (R.fused) FQ_TRY(reduce_partials(ctx, gb2, grid, ctx->d_result + dst_b2));
+            FQ_TRY(reduce_partials(ctx, gb, grid, ctx->result + dst_b));
+            if (energy_here) FQ_TRY(reduce_partials(ctx, gg, grid, ctx->result));
+            if (R.phi) FQ_TRY(reduce_partials(ctx, gg, grid, ctx->result + dst_g));
+            if (R.fused) FQ_TRY(reduce_partials(ctx, gb2, grid, ctx->result + dst_b2));
         }
     }
     if (batched) {
         const int tok = prof_begin(ctx);
         k_reduce_grad<<<3 * nrev, 256, 0, ctx->stream>>>(ctx->d_partial, grid, sums,
-                                                         ctx->d_result);
+                                                         ctx->result);
         FQ_CUDA(cudaGetLastError());
         prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
         ctx->launches++;
     }
-    FQ_CUDA(cudaMemcpyAsync(ctx->h_result, ctx->d_result, sizeof(double) * (1 + P + P * npass),
-                            cudaMemcpyDeviceToHost, ctx->stream));
-    // The kernels' error flag travels with the results (last result word).
-    FQ_CUDA(cudaMemcpyAsync(ctx->h_result + kResultWords - 1, ctx->d_err, sizeof(int),
-                            cudaMemcpyDeviceToHost, ctx->stream));
     return FQ_OK;
 }
 
 int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,
                  double* grad_beta) {
-    const bool half = half_state(N);
-    const double m = half ? 2.0 : 1.0;  // the sums of a half state are half the whole
-    const int npass = (int)plan_layer(N, half).size();
-    const double* r = ctx->h_result;
-    int flag = 0;
-    memcpy(&flag, r + kResultWords - 1, sizeof(int));
-    if (flag) {
-        FQ_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(int), ctx->stream));
-        set_error("a device-side bounded wait gave up (flag %d); results are incomplete", flag);
-        return FQ_ERR_TIMEOUT;
+    const double m = 2.0;  // the sums of a half state are half the whole
+    const int npass = (int)plan_layer(N, true).size();
+    const double* r = ctx->result;
+    FQ_TRY(check_device_error(ctx));
+    if (N <= kSmallKernelQubits) {  // run_small's results
+        *energy = r[0];
+        std::copy(r + 1, r + 1 + P, grad_gamma);
+        std::copy(r + 1 + P, r + 1 + 2 * P, grad_beta);
+        return FQ_OK;
     }
     *energy = m * r[0];
     for (int k = 0; k < P; k++) {
@@ -363,18 +238,10 @@ int fq_qaoa_energy_grad(fq_ctx* ctx, void* sv, void* costate, int N, int P, cons
         FQ_CHECK(1 + 2 * P <= kResultWords, FQ_ERR_INVALID, "P=%d too large", P);
         GraphPrep g;
         FQ_TRY(prep_graph(graph, N, g));
-        SmallHostJob J{N, P, SJ_ENERGY | SJ_GRAD, g.wd.data(), gammas, betas, nullptr};
-        std::vector<int> off;
-        FQ_TRY(run_small_jobs(ctx, &J, 1, 0, off));
-        FQ_TRY(read_results(ctx, 1 + 2 * P));
-        *energy = ctx->h_result[0];
-        for (int k = 0; k < P; k++) {
-            grad_gamma[k] = ctx->h_result[1 + k];
-            grad_beta[k] = ctx->h_result[1 + P + k];
-        }
-        return FQ_OK;
+        FQ_TRY(run_small(ctx, g, P, gammas, betas, SJ_GRAD, nullptr, ctx->result));
+    } else {
+        FQ_TRY(grad_enqueue(ctx, sv, costate, N, P, graph, gammas, betas));
     }
-    FQ_TRY(grad_enqueue(ctx, sv, costate, N, P, graph, gammas, betas));
     FQ_CUDA(cudaStreamSynchronize(ctx->stream));
     return grad_collect(ctx, N, P, energy, grad_gamma, grad_beta);
 }

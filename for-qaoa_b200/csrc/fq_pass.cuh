@@ -33,8 +33,8 @@
 //
 // Half states.  A circuit from |+>^N keeps psi(~z) = psi(z): the start, the
 // cut phase (C(~z) = C(z)) and RX on every qubit commute with flipping all
-// bits, and so does lambda = C psi.  The engine's circuits and gradients of
-// N >= 13 qubits therefore sweep only the 2^(N-1) amplitudes with qubit N-1
+// bits, and so does lambda = C psi.  The engine's circuits and gradients
+// therefore sweep only the 2^(N-1) amplitudes with qubit N-1
 // = 0, half the traffic and half the arithmetic.  An amplitude z with qubit
 // N-1 set is stored at ~z.  Strided tiles over qubits 11..N-2 are those of
 // the whole state with that bit 0; the contiguous pass becomes the mirror
@@ -43,7 +43,7 @@
 // mirrored addresses 2^(N-1) - 1 - x (two runs of 2048 contiguous
 // amplitudes, one walked backwards).  Phases, cut constants and rotations
 // see an ordinary tile of the N-qubit state.  The pass that ends a forward
-// circuit writes both halves (ST = 2).  Measured: half_state, fq_engine.h.
+// circuit writes both halves (ST = 2).  Measured: engine_args, fq_engine.h.
 //
 // Cut value of an amplitude (exact in integers for integer weights):
 //   C(z) = K(fixed) + C_TT(tile bits) + sum_{u in tile} z_u e_u(fixed)

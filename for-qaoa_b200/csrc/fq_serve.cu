@@ -4,12 +4,11 @@
 // GPU; a scheduler thread runs the small-instance batches and every lane has
 // a thread of its own, so the ~30 kernel launches of a larger request are
 // issued by its lane's thread, in parallel with the other lanes':
-//   - small instances (N <= 15) are packed into launches of k_small_jobs,
-//     the whole instance in shared memory: one CTA each up to 12 qubits, a
-//     cluster of 2^(N-12) CTAs above (distributed shared memory), one launch
-//     per size class; two batches can be in flight on their own streams,
-//     and a batch takes every small request queued when it launches (up to
-//     its capacity);
+//   - small instances (N <= 15) are packed into launches of the small-instance
+//     kernels (fq_small.cuh): one CTA each up to 13 qubits, a cluster of
+//     2^(N-13) CTAs above, one launch per size class, side by side on streams
+//     of their own; two batches can be in flight, and a batch takes every
+//     small request queued when it launches (up to its capacity);
 //   - larger instances run on lanes (an fq_ctx each: its own stream and
 //     scratch), so independent requests overlap; a free lane takes the
 //     oldest queued request whose session is idle and whose buffers are
@@ -53,7 +52,8 @@ size_t session_bytes(int N) { return 2 * (sizeof(double2) << N); }
 struct Req {
     uint64_t ticket = 0, session = 0;
     int N = 0, P = 0;
-    std::vector<double> w;      // N*N symmetric (small instances)
+    SmallJob job;               // small instances: descriptor and data words
+    std::vector<double> data;
     std::vector<double> graph;  // N*N upper triangle (large instances)
     std::vector<double> gammas, betas;
     double t_submit = 0, t_start = 0;
@@ -103,10 +103,13 @@ constexpr int kBatchOut = kBatchCap * (1 + 2 * FQ_SERVE_MAX_LAYERS);
 struct Batch {
     cudaStream_t st = nullptr;
     cudaEvent_t done = nullptr;
+    // Size classes run side by side: the batch's stream carries the upload,
+    // every class but the first present forks from it (to the server's stream
+    // of its class) and joins it again.
+    cudaEvent_t up = nullptr, joined[kSmallClasses] = {};
     unsigned char* h_in = nullptr;  // pinned
     unsigned char* d_in = nullptr;
-    double* h_out = nullptr;  // pinned
-    double* d_out = nullptr;
+    double* out = nullptr;  // pinned, written by the kernels
     std::vector<Req> reqs;
     std::vector<int> out_off;
     bool busy = false;
@@ -127,6 +130,7 @@ struct fq_server {
     cudaStream_t free_stream = nullptr;
     std::vector<Lane> lanes;
     Batch batches[2];
+    cudaStream_t side[kSmallClasses] = {};  // of both batches
     std::map<uint64_t, Session> sessions;  // guarded by mu
     std::deque<Req> small_q, large_q;      // guarded by mu
     std::vector<fq_result> done;           // guarded by mu
@@ -177,21 +181,17 @@ struct fq_server {
 
     // ---- small instances (one CTA each, or one cluster of CTAs) --------------
     static size_t job_bytes(const Req& r) {
-        return sizeof(SmallJob) + sizeof(double) * (r.N * r.N + 2 * r.P);
+        return sizeof(SmallJob) + sizeof(double) * r.data.size();
     }
 
     int launch_batch(Batch& B) {
         const int nj = (int)B.reqs.size();
-        // One launch per size class (one CTA, clusters of 2, 4, 8 CTAs):
-        // the batch in class order.
+        // One launch per size class: the batch in class order.
         std::stable_sort(B.reqs.begin(), B.reqs.end(), [](const Req& a, const Req& b) {
             return small_class(a.N) < small_class(b.N);
         });
-        int nmax = 1, counts[kSmallClasses] = {};
-        for (auto& r : B.reqs) {
-            counts[small_class(r.N)]++;
-            if (small_class(r.N) == 0) nmax = std::max(nmax, r.N);
-        }
+        int counts[kSmallClasses] = {};
+        for (auto& r : B.reqs) counts[small_class(r.N)]++;
         SmallJob* hj = reinterpret_cast<SmallJob*>(B.h_in);
         double* hd = reinterpret_cast<double*>(B.h_in + sizeof(SmallJob) * nj);
         const double* dd = reinterpret_cast<const double*>(B.d_in + sizeof(SmallJob) * nj);
@@ -200,31 +200,41 @@ struct fq_server {
         B.out_off.assign(nj, 0);
         for (int i = 0; i < nj; i++) {
             const Req& r = B.reqs[i];
-            SmallJob d;
-            d.N = r.N;
-            d.P = r.P;
-            d.flags = SJ_ENERGY | SJ_GRAD;
-            d.pad = 0;
-            memcpy(hd + off, r.w.data(), sizeof(double) * r.N * r.N);
+            SmallJob d = r.job;
+            memcpy(hd + off, r.data.data(), sizeof(double) * r.data.size());
             d.w = dd + off;
-            off += r.N * r.N;
-            memcpy(hd + off, r.gammas.data(), sizeof(double) * r.P);
-            d.gammas = dd + off;
-            off += r.P;
-            memcpy(hd + off, r.betas.data(), sizeof(double) * r.P);
-            d.betas = dd + off;
-            off += r.P;
-            d.out = B.d_out + o;
+            d.lay = d.w + r.N * (r.N - 1) / 2;
+            off += r.data.size();
+            d.out = B.out + o;
             B.out_off[i] = o;
             o += 1 + 2 * r.P;
-            d.state = nullptr;
             hj[i] = d;
         }
         const size_t need = sizeof(SmallJob) * nj + sizeof(double) * off;
         FQ_CUDA(cudaMemcpyAsync(B.d_in, B.h_in, need, cudaMemcpyHostToDevice, B.st));
-        FQ_TRY(launch_small_jobs(reinterpret_cast<const SmallJob*>(B.d_in), counts, nmax, B.st));
-        FQ_CUDA(cudaMemcpyAsync(B.h_out, B.d_out, sizeof(double) * o, cudaMemcpyDeviceToHost,
-                                B.st));
+        FQ_CUDA(cudaEventRecord(B.up, B.st));
+        const SmallJob* dj = reinterpret_cast<const SmallJob*>(B.d_in);
+        // The largest class first, on the batch's own stream.
+        bool first = true;
+        int at = nj, st = FQ_OK;
+        for (int c = kSmallClasses - 1; c >= 0; c--) {
+            at -= counts[c];
+            if (counts[c] == 0) continue;
+            cudaStream_t s = first ? B.st : side[c];
+            if (!first && cudaStreamWaitEvent(s, B.up, 0) != cudaSuccess) st = FQ_ERR_CUDA;
+            if (st == FQ_OK) st = launch_small_batch(dj + at, counts[c], c, s);
+            if (!first && (cudaEventRecord(B.joined[c], s) != cudaSuccess ||
+                           cudaStreamWaitEvent(B.st, B.joined[c], 0) != cudaSuccess) &&
+                st == FQ_OK)
+                st = FQ_ERR_CUDA;
+            first = false;
+        }
+        if (st != FQ_OK) {
+            // What was launched is done with the buffers before they are reused.
+            for (int c = 0; c < kSmallClasses; c++) cudaStreamSynchronize(side[c]);
+            cudaStreamSynchronize(B.st);
+            return st;
+        }
         FQ_CUDA(cudaEventRecord(B.done, B.st));
         B.busy = true;
         B.t_start = now_s();
@@ -236,7 +246,7 @@ struct fq_server {
     void complete_batch(Batch& B) {
         for (size_t i = 0; i < B.reqs.size(); i++) {
             const Req& r = B.reqs[i];
-            const double* out = B.h_out + B.out_off[i];
+            const double* out = B.out + B.out_off[i];
             finish(r, FQ_OK, out, out + 1, out + 1 + r.P, B.t_start);
         }
         B.reqs.clear();
@@ -500,10 +510,17 @@ int fq_server_create(int device, double hbm_budget_bytes, int lanes, fq_server**
             cudaEventCreateWithFlags(&B.done, cudaEventDisableTiming) != cudaSuccess ||
             cudaMallocHost(&B.h_in, kBatchBytes) != cudaSuccess ||
             cudaMalloc(&B.d_in, kBatchBytes) != cudaSuccess ||
-            cudaMallocHost(&B.h_out, sizeof(double) * kBatchOut) != cudaSuccess ||
-            cudaMalloc(&B.d_out, sizeof(double) * kBatchOut) != cudaSuccess)
+            cudaEventCreateWithFlags(&B.up, cudaEventDisableTiming) != cudaSuccess ||
+            cudaMallocHost(&B.out, sizeof(double) * kBatchOut) != cudaSuccess)
             st = FQ_ERR_OOM;
+        for (int c = 0; c < kSmallClasses && st == FQ_OK; c++)
+            if (cudaEventCreateWithFlags(&B.joined[c], cudaEventDisableTiming) != cudaSuccess)
+                st = FQ_ERR_CUDA;
     }
+    for (int c = 0; c < kSmallClasses && st == FQ_OK; c++)
+        if (cudaStreamCreateWithPriority(&S->side[c], cudaStreamNonBlocking, prio_high) !=
+            cudaSuccess)
+            st = FQ_ERR_CUDA;
     if (st == FQ_OK) {
         // A pool of its own that keeps freed session buffers for reuse.
         cudaMemPoolProps props;
@@ -567,9 +584,13 @@ int fq_server_destroy(fq_server* S) {
         if (B.st) cudaStreamDestroy(B.st);
         if (B.h_in) cudaFreeHost(B.h_in);
         cudaFree(B.d_in);
-        if (B.h_out) cudaFreeHost(B.h_out);
-        cudaFree(B.d_out);
+        if (B.out) cudaFreeHost(B.out);
+        if (B.up) cudaEventDestroy(B.up);
+        for (cudaEvent_t e : B.joined)
+            if (e) cudaEventDestroy(e);
     }
+    for (cudaStream_t s : S->side)
+        if (s) cudaStreamDestroy(s);
     delete S;
     return FQ_OK;
 }
@@ -593,10 +614,12 @@ int fq_server_submit(fq_server* S, const fq_request* q, uint64_t* ticket) {
     r.gammas.assign(q->gammas, q->gammas + q->P);
     r.betas.assign(q->betas, q->betas + q->P);
     const bool small = q->N <= kSmallJobMaxQubits;
-    if (small)
-        r.w = g.wd;
-    else
+    if (small) {
+        r.data.resize(small_words(q->N, q->P));
+        small_job(g, q->P, q->gammas, q->betas, SJ_GRAD, false, r.job, r.data.data());
+    } else {
         r.graph.assign(q->graph_upper, q->graph_upper + (size_t)q->N * q->N);
+    }
     r.t_submit = now_s();
     std::lock_guard<std::mutex> lk(S->mu);
     FQ_CHECK(!S->stop, FQ_ERR_INVALID, "the server is stopping");

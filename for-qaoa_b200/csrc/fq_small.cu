@@ -1,0 +1,164 @@
+// fq_small.cu -- host side of the small-instance kernels (fq_small.cuh): one
+// instance with its data in the kernel parameters, or batches of one size
+// class.
+#include <math.h>
+#include <string.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "fq_ctx.h"
+#include "fq_engine.h"
+#include "fq_small.cuh"
+
+namespace fq {
+
+void small_job(const GraphPrep& g, int P, const double* gammas, const double* betas, int flags,
+               bool alone, SmallJob& J, double* data) {
+    const int N = g.N;
+    memset(&J, 0, sizeof(J));
+    J.N = N;
+    J.P = P;
+    J.flags = flags;
+    const long long range = g.cmax - g.cmin + 1;
+    // A table where it takes fewer sincos (half its entries) than the 2^(N-1)
+    // amplitudes do, and fits.
+    const int cap = small_table_cap(small_class(N), alone);
+    J.ntab = g.integer && range <= cap && range <= 1ll << N ? (int)range : 0;
+    J.keep = J.ntab > 0 && (long long)P * range <= cap;
+    J.cmin = (int)g.cmin;
+    J.W = g.W;
+    for (int i = 0; i < N; i++)
+        for (int j = i + 1; j < N; j++) *data++ = g.wd[i * N + j];
+    int cot = 0;
+    for (int p = 0; p < P; p++) {
+        int gm;
+        double gx, f;
+        gate_params(betas[p], gm, gx, f);
+        cot += gm != GM_TAN;
+        *data++ = gammas[p];
+        *data++ = gm == GM_TAN ? gx : -gx;
+        *data++ = pow(f, N) * (p == 0 ? fq_init_amp(N) : 1.0);
+        *data++ = f * f;
+    }
+    J.rot = (int)((long long)N * cot & 3);
+}
+
+namespace {
+
+// The largest of the one-CTA classes, which share their kernels.
+size_t small_smem_max(bool grad) {
+    size_t m = 0;
+    for (int c = 0; c <= 4; c++) m = std::max(m, small_smem_bytes(c, grad, true));
+    return m;
+}
+
+template <typename Fn>
+int launch_cluster(Fn fn, int cb, int njobs, size_t smem, cudaStream_t st, void** args) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)njobs << cb);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 1u << cb;
+    at.val.clusterDim.y = 1;
+    at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    FQ_CUDA(cudaLaunchKernelExC(&cfg, (const void*)fn, args));
+    return FQ_OK;
+}
+
+// One size class C (small_class): a single instance (one != null) or njobs
+// descriptors on the device.
+template <int C, bool GRAD>
+int launch_class(const SmallArgs* one, const SmallJob* jobs, int njobs, cudaStream_t st) {
+    void* args[1] = {one ? (void*)one : (void*)&jobs};
+    if constexpr (C <= 4) {
+        const size_t smem = small_smem_bytes(C, GRAD, one != nullptr);
+        const void* fn = one ? (const void*)k_small_one<GRAD> : (const void*)k_small_batch<GRAD>;
+        // Every class shares the function, and threads set this concurrently:
+        // always the largest class's size.
+        FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)small_smem_max(GRAD)));
+        // A warp at least; one instance alone also gets warps that only help
+        // to fill the phase tables.
+        const int threads = std::max(32 << C, one ? 256 : 32);
+        FQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)njobs), dim3(threads), args, smem, st));
+        return FQ_OK;
+    } else {
+        constexpr int CB = C - 4;
+        const size_t smem = small_cluster_smem_bytes(GRAD);
+        const void* fn = one ? (const void*)k_small_cluster_one<CB, GRAD>
+                             : (const void*)k_small_cluster_batch<CB, GRAD>;
+        FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return launch_cluster(fn, CB, njobs, smem, st, args);
+    }
+}
+
+template <bool GRAD>
+int launch_any(int c, const SmallArgs* one, const SmallJob* jobs, int njobs, cudaStream_t st) {
+    switch (c) {
+        case 0: return launch_class<0, GRAD>(one, jobs, njobs, st);
+        case 1: return launch_class<1, GRAD>(one, jobs, njobs, st);
+        case 2: return launch_class<2, GRAD>(one, jobs, njobs, st);
+        case 3: return launch_class<3, GRAD>(one, jobs, njobs, st);
+        case 4: return launch_class<4, GRAD>(one, jobs, njobs, st);
+        case 5: return launch_class<5, GRAD>(one, jobs, njobs, st);
+        case 6: return launch_class<6, GRAD>(one, jobs, njobs, st);
+        default: return launch_class<7, GRAD>(one, jobs, njobs, st);
+    }
+}
+
+}  // namespace
+
+int launch_small_batch(const SmallJob* jobs, int njobs, int c, cudaStream_t st) {
+    return launch_any<true>(c, nullptr, jobs, njobs, st);
+}
+
+int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
+              int flags, double2* state, double* out) {
+    const int c = small_class(g.N), words = small_words(g.N, P);
+    const bool grad = flags & SJ_GRAD;
+    const int tok = prof_begin(ctx);
+    if (words <= kSmallArgWords) {
+        SmallArgs a;
+        small_job(g, P, gammas, betas, flags, true, a.job, a.data);
+        a.job.out = out;
+        a.job.state = state;
+        FQ_TRY(grad ? launch_any<true>(c, &a, nullptr, 1, ctx->stream)
+                    : launch_any<false>(c, &a, nullptr, 1, ctx->stream));
+    } else {
+        // Deep circuits: descriptor and data through device memory.
+        std::vector<double> h((sizeof(SmallJob) + 7) / 8 + words);
+        double* const data = h.data() + (h.size() - words);
+        SmallJob J;
+        small_job(g, P, gammas, betas, flags, false, J, data);
+        void* d = nullptr;
+        FQ_CUDA(cudaMalloc(&d, h.size() * sizeof(double)));
+        J.w = (const double*)d + (h.size() - words);
+        J.lay = J.w + g.N * (g.N - 1) / 2;
+        J.out = out;
+        J.state = state;
+        memcpy(h.data(), &J, sizeof(J));
+        int st = FQ_OK;
+        if (cudaMemcpyAsync(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice,
+                            ctx->stream) != cudaSuccess)
+            st = FQ_ERR_CUDA;
+        if (st == FQ_OK)
+            st = grad ? launch_any<true>(c, nullptr, (const SmallJob*)d, 1, ctx->stream)
+                      : launch_any<false>(c, nullptr, (const SmallJob*)d, 1, ctx->stream);
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        cudaFree(d);
+        FQ_TRY(st);
+        FQ_CUDA(e);
+    }
+    prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
+    ctx->launches++;
+    return FQ_OK;
+}
+
+}  // namespace fq

@@ -1,41 +1,50 @@
-// fq_small.h -- job descriptor of k_small_jobs (fq_small.cuh): one whole
-// QAOA instance of up to 12 qubits per CTA, of 13..15 qubits per cluster of
-// 2^(N-12) CTAs.
+// fq_small.h -- job descriptor of the small-instance kernels (fq_small.cuh):
+// one whole QAOA instance per CTA (N <= 13) or per cluster of 2^(N-13) CTAs
+// (N = 14..16).
 #pragma once
+
+#include <vector>
 
 #include "fq_common.cuh"
 
 namespace fq {
 
-constexpr int kSmallMaxQubits = 12;     // qubits held by one CTA
-constexpr int kSmallJobMaxQubits = 15;  // qubits of a job (a cluster of up to 8 CTAs)
-constexpr int kSmallThreads = 256;
+constexpr int kSmallMaxQubits = 13;     // qubits of a one-CTA instance
+constexpr int kSmallJobMaxQubits = 15;  // qubits of a request that needs no buffers (FQ_SMALL_MAX_QUBITS)
+constexpr int kSmallKernelQubits = 16;  // qubits of the largest instance a cluster holds
 
-enum { SJ_ENERGY = 1, SJ_GRAD = 2, SJ_STATE = 4 };
+enum { SJ_GRAD = 1, SJ_STATE = 2 };
 
 struct SmallJob {
-    int N, P, flags, pad;
-    const double* w;       // N*N symmetric weights (device)
-    const double* gammas;  // P (device)
-    const double* betas;   // P (device)
-    double* out;           // [0] <C>, [1..P] dE/dgamma, [1+P..2P] dE/dbeta (device)
-    double2* state;        // final forward state (SJ_STATE), 2^N (device)
+    int N, P, flags;
+    int ntab;           // integer weights: cut values cmin..cmin+ntab-1 get a phase table; 0: sincos
+    int keep;           // every layer's table is kept (P * ntab entries), else one at a time
+    int cmin;
+    int rot;            // the final state is (-i)^rot times what the layers give (see small_job)
+    double W;           // total weight
+    const double* w;    // upper triangle, row by row: N(N-1)/2
+    const double* lay;  // 4 per layer: gamma, t, the phase's scale, f^2
+    double* out;        // [0] <C>, then with SJ_GRAD dE/dgamma[P], dE/dbeta[P]
+    double2* state;     // final state (SJ_STATE), 2^N
 };
 
-// Shared memory of a CTA holding 2^nl amplitudes: psi, lambda, the cut
-// values, the weights of a job of up to kSmallJobMaxQubits qubits, the
-// block-sum scratch and the cluster's exchange words.
-// Size class of an N-qubit job: 0 for one CTA (N <= 12), else the log2 of
-// its cluster's CTAs.
-constexpr int kSmallClasses = kSmallJobMaxQubits - kSmallMaxQubits + 1;
-__host__ __device__ inline int small_class(int N) {
-    return N <= kSmallMaxQubits ? 0 : N - kSmallMaxQubits;
-}
+// Data words of a job behind its descriptor.
+__host__ __device__ inline int small_words(int N, int P) { return N * (N - 1) / 2 + 4 * P; }
 
-__host__ __device__ inline size_t small_smem_bytes(int nl) {
-    const size_t n = (size_t)1 << nl;
-    return 2 * n * sizeof(double2) + n * sizeof(double) +
-           sizeof(double) * (kSmallJobMaxQubits * kSmallJobMaxQubits + kSmallThreads + 8);
+// Size class of an N-qubit instance: 0..4 for one CTA of 2^(8..12)
+// amplitudes (a half state from N = 9 on), 5..7 for clusters of 2, 4, 8.
+constexpr int kSmallClasses = 8;
+__host__ __device__ inline int small_class(int N) {
+    return N <= 9 ? 0 : N <= kSmallMaxQubits ? N - 9 : N - kSmallMaxQubits + 4;
+}
+// Phase-table entries of a job of size class c: what is left of the shared
+// memory at the residency its registers allow in a batch (4 CTAs per SM and
+// more up to class 2, two of class 3, one of class 4), and more for an
+// instance alone.  Clusters use the room integer cut values leave free.
+__host__ __device__ inline int small_table_cap(int c, bool alone) {
+    if (c > 4) return 2048;
+    if (c == 4) return 2816;
+    return alone ? 4096 : 128 << c;
 }
 
 }  // namespace fq
