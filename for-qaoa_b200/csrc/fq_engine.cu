@@ -89,10 +89,6 @@ __global__ void k_reduce_partials(const double* partial, int n, double* out) {
     if (threadIdx.x == 0) out[0] = sh[0];
 }
 
-struct Perm {
-    int p[kMaxQubits];
-};
-
 // Per-block max|a-b|^2, max|b|^2, sum|a-b|^2, sum|b|^2 over a grid-stride
 // split (fixed per launch geometry, so the same inputs give the same bits).
 __global__ void k_state_diff(const double2* a, const double2* b, u64 n, double* part) {
@@ -122,17 +118,6 @@ __global__ void k_state_diff(const double2* a, const double2* b, u64 n, double* 
         __syncthreads();
     }
     if (threadIdx.x < 4) part[4 * blockIdx.x + threadIdx.x] = sh[threadIdx.x][0];
-}
-
-__global__ void k_permute(const double2* __restrict__ src, double2* __restrict__ dst, int N,
-                          Perm P) {
-    const u64 n = 1ull << N;
-    for (u64 x = blockIdx.x * (u64)blockDim.x + threadIdx.x; x < n;
-         x += (u64)gridDim.x * blockDim.x) {
-        u64 y = 0;
-        for (int b = 0; b < N; b++) y |= ((x >> b) & 1ull) << P.p[b];
-        dst[y] = src[x];
-    }
 }
 
 // Small states (N < 12, at most 2048 amplitudes): one CTA, the reference's
@@ -840,28 +825,6 @@ int fq_rx_targets(fq_ctx* ctx, void* sv, int N, const int* targets, int n, doubl
         seen |= 1ull << t;
     }
     return rx_mask(ctx, sv, N, seen, angle);
-}
-
-int fq_permute_qubits(fq_ctx* ctx, const void* src, void* dst, int N, const int* perm) {
-    FQ_TRY(validate_ctx(ctx));
-    FQ_TRY(check_state((void*)src, N));
-    FQ_TRY(check_state(dst, N));
-    FQ_CHECK(src != dst, FQ_ERR_INVALID, "permutation must be out of place");
-    FQ_CHECK(perm != nullptr, FQ_ERR_INVALID, "null permutation");
-    Perm P;
-    unsigned long long seen = 0;
-    for (int b = 0; b < N; b++) {
-        FQ_CHECK(perm[b] >= 0 && perm[b] < N && !((seen >> perm[b]) & 1ull), FQ_ERR_INVALID,
-                 "perm is not a permutation of 0..N-1");
-        seen |= 1ull << perm[b];
-        P.p[b] = perm[b];
-    }
-    const u64 n = 1ull << N;
-    const unsigned grid = (unsigned)std::min<u64>((n + 255) / 256, (u64)ctx->num_sms * 16);
-    k_permute<<<grid, 256, 0, ctx->stream>>>((const double2*)src, (double2*)dst, N, P);
-    FQ_CUDA(cudaGetLastError());
-    ctx->launches++;
-    return FQ_OK;
 }
 
 int fq_state_diff(fq_ctx* ctx, const void* a, const void* b, int N, double* out) {
