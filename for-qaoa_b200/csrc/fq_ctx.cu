@@ -31,6 +31,7 @@ int check_device_error(fq_ctx* ctx) {
     const int flag = *(volatile int*)ctx->err;
     if (flag) {
         *(volatile int*)ctx->err = 0;
+        ctx->counter_lost = true;
         set_error("a device-side bounded wait gave up (flag %d); results are incomplete", flag);
         return FQ_ERR_TIMEOUT;
     }
@@ -196,20 +197,27 @@ int fq_ctx_create(int device, void* stream, fq_ctx** out) {
             }
             c->own_stream = true;
         }
-        cudaDeviceProp prop;
-        if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) { st = FQ_ERR_CUDA; break; }
-        c->num_sms = prop.multiProcessorCount;
+        int coop = 0;
+        if (cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device) !=
+                cudaSuccess ||
+            cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess) {
+            st = FQ_ERR_CUDA;
+            break;
+        }
+        c->cooperative = coop != 0;
         c->partial_cap = 256 * c->num_sms;  // room for every pass of a gradient's reverse sweep
         const size_t wbytes = sizeof(double) * kMaxQubits * kMaxQubits;
         if (cudaMalloc(&c->d_w, wbytes) != cudaSuccess ||
             cudaMalloc(&c->d_ptab, sizeof(double2) * kMaxPhaseTable) != cudaSuccess ||
             cudaMalloc(&c->d_partial, sizeof(double) * c->partial_cap) != cudaSuccess ||
             cudaMalloc(&c->d_tcut, kTcutBytes) != cudaSuccess ||
-            cudaMalloc(&c->d_img, kMaxGeoms * kImgStride) != cudaSuccess) {
+            cudaMalloc(&c->d_img, kMaxGeoms * kImgStride) != cudaSuccess ||
+            cudaMalloc(&c->d_counter, sizeof(unsigned)) != cudaSuccess) {
             st = FQ_ERR_OOM;
             break;
         }
         c->tcut_bytes = kTcutBytes;
+        c->counter_lost = true;  // zeroed by the first launch that uses it
         c->h_stage_bytes = std::max(wbytes, (size_t)256 * 1024);
         if (cudaMallocHost(&c->h_stage, c->h_stage_bytes) != cudaSuccess ||
             cudaMallocHost(&c->result, sizeof(double) * kResultWords + 64) != cudaSuccess) {
@@ -242,6 +250,7 @@ int fq_ctx_destroy(fq_ctx* c) {
     cudaFree(c->d_partial);
     cudaFree(c->d_tcut);
     cudaFree(c->d_img);
+    cudaFree(c->d_counter);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->result) cudaFreeHost(c->result);
     if (c->stage_evt) cudaEventDestroy(c->stage_evt);

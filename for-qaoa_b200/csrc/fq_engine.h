@@ -88,13 +88,19 @@ int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,
 // Small instances (fq_small.cuh, N <= kSmallKernelQubits).  small_job fills a
 // descriptor (its pointers apart) and its small_words(N, P) data words: the
 // weights, then the layers.
-// alone: the job is launched by itself (run_small), not in a batch.
+// cap: phase-table entries there is room for; most: entries of one layer's
+// table that are worth computing.
 void small_job(const GraphPrep& g, int P, const double* gammas, const double* betas, int flags,
-               bool alone, SmallJob& J, double* data);
+               int cap, long long most, SmallJob& J, double* data);
 // Enqueues one instance on ctx's stream; out (1 + 2P words with SJ_GRAD,
 // else 1) and state (SJ_STATE) are device-accessible.
 int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
               int flags, double2* state, double* out);
+// One whole circuit or gradient (SJ_STATE or SJ_GRAD) of 16..19 qubits as a
+// cooperative launch (fq_mid.cuh), where mid_ok says so; results as run_small's.
+bool mid_ok(const fq_ctx* ctx, int N, int P);
+int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
+            int flags, double2* state, double2* lam, double* out);
 // Gradients of njobs instances of size class c, descriptors on the device.
 int launch_small_batch(const SmallJob* jobs, int njobs, int c, cudaStream_t stream);
 

@@ -616,7 +616,8 @@ int fq_server_submit(fq_server* S, const fq_request* q, uint64_t* ticket) {
     const bool small = q->N <= kSmallJobMaxQubits;
     if (small) {
         r.data.resize(small_words(q->N, q->P));
-        small_job(g, q->P, q->gammas, q->betas, SJ_GRAD, false, r.job, r.data.data());
+        small_job(g, q->P, q->gammas, q->betas, SJ_GRAD, small_table_cap(small_class(q->N), false),
+                  small_table_most(q->N), r.job, r.data.data());
     } else {
         r.graph.assign(q->graph_upper, q->graph_upper + (size_t)q->N * q->N);
     }

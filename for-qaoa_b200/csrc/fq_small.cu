@@ -9,22 +9,19 @@
 
 #include "fq_ctx.h"
 #include "fq_engine.h"
-#include "fq_small.cuh"
+#include "fq_mid.cuh"
 
 namespace fq {
 
 void small_job(const GraphPrep& g, int P, const double* gammas, const double* betas, int flags,
-               bool alone, SmallJob& J, double* data) {
+               int cap, long long most, SmallJob& J, double* data) {
     const int N = g.N;
     memset(&J, 0, sizeof(J));
     J.N = N;
     J.P = P;
     J.flags = flags;
     const long long range = g.cmax - g.cmin + 1;
-    // A table where it takes fewer sincos (half its entries) than the 2^(N-1)
-    // amplitudes do, and fits.
-    const int cap = small_table_cap(small_class(N), alone);
-    J.ntab = g.integer && range <= cap && range <= 1ll << N ? (int)range : 0;
+    J.ntab = g.integer && range <= cap && range <= most ? (int)range : 0;
     J.keep = J.ntab > 0 && (long long)P * range <= cap;
     J.cmin = (int)g.cmin;
     J.W = g.W;
@@ -119,6 +116,50 @@ int launch_small_batch(const SmallJob* jobs, int njobs, int c, cudaStream_t st) 
     return launch_any<true>(c, nullptr, jobs, njobs, st);
 }
 
+// Amplitude bits per CTA: 128 CTAs, as small as two warps.  On B200, gradient
+// p=6 with 9, 10, 11, 12 bits: N=16 107, 117, 141, 189 us; N=18 124
+// with 10, 150, 202; N=19 148 with 11, 206 with 12.
+static int mid_bits(int N) { return std::max(kMidMinBits, N - 8); }
+
+bool mid_ok(const fq_ctx* ctx, int N, int P) {
+    return N >= kMidMinQubits && N <= kMidMaxQubits && P <= kMidMaxLayers &&
+           1 << (N - 1 - mid_bits(N)) <= ctx->num_sms && ctx->cooperative;
+}
+
+int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
+            int flags, double2* state, double2* lam, double* out) {
+    const int N = g.N, nb = mid_bits(N), grid = 1 << (N - 1 - nb), threads = 1 << (nb - kSmallBits);
+    const bool grad = flags & SJ_GRAD;
+    MidArgs a;
+    a.nb = nb;
+    small_job(g, P, gammas, betas, flags, kMidTable, 16 * threads, a.job, a.data);
+    a.job.out = out;
+    a.job.state = state;
+    a.lam = lam;
+    a.partial = ctx->d_partial;
+    a.counter = ctx->d_counter;
+    a.err = ctx->err;
+    if (ctx->counter_lost) {  // a barrier gave up: its arrivals are not all counted
+        FQ_CUDA(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
+        ctx->counter_base = 0;
+        ctx->counter_lost = false;
+    }
+    a.base = ctx->counter_base;
+    const void* fn = grad ? (const void*)k_mid<true> : (const void*)k_mid<false>;
+    const size_t smem = mid_smem_bytes(nb, grad);
+    // The largest size for every N: contexts on other threads set it too.
+    FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)mid_smem_bytes(kMidMaxBits, grad)));
+    void* args[1] = {&a};
+    const int tok = prof_begin(ctx);
+    FQ_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem,
+                                        ctx->stream));
+    prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
+    ctx->counter_base += (unsigned)(((grad ? 2 : 1) * P + 1) * grid);  // its barriers
+    ctx->launches++;
+    return FQ_OK;
+}
+
 int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
               int flags, double2* state, double* out) {
     const int c = small_class(g.N), words = small_words(g.N, P);
@@ -126,7 +167,8 @@ int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, cons
     const int tok = prof_begin(ctx);
     if (words <= kSmallArgWords) {
         SmallArgs a;
-        small_job(g, P, gammas, betas, flags, true, a.job, a.data);
+        small_job(g, P, gammas, betas, flags, small_table_cap(c, true), small_table_most(g.N), a.job,
+                  a.data);
         a.job.out = out;
         a.job.state = state;
         FQ_TRY(grad ? launch_any<true>(c, &a, nullptr, 1, ctx->stream)
@@ -136,7 +178,8 @@ int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, cons
         std::vector<double> h((sizeof(SmallJob) + 7) / 8 + words);
         double* const data = h.data() + (h.size() - words);
         SmallJob J;
-        small_job(g, P, gammas, betas, flags, false, J, data);
+        small_job(g, P, gammas, betas, flags, small_table_cap(c, false), small_table_most(g.N), J,
+                  data);
         void* d = nullptr;
         FQ_CUDA(cudaMalloc(&d, h.size() * sizeof(double)));
         J.w = (const double*)d + (h.size() - words);

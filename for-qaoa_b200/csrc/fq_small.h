@@ -47,4 +47,7 @@ __host__ __device__ inline int small_table_cap(int c, bool alone) {
     return alone ? 4096 : 128 << c;
 }
 
+// A table is worth its sincos (half its entries) up to the 2^(N-1) amplitudes.
+inline long long small_table_most(int N) { return 1ll << N; }
+
 }  // namespace fq

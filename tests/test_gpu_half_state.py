@@ -1,9 +1,9 @@
-"""GPU parity of whole circuits and gradients on half states (N >= 17: only
-the amplitudes with qubit N-1 = 0 are swept, the last pass writes both
-halves) at the edges of their tile geometries: rows of 64 to 16 amplitudes
-(N=17..20), paired rows of 8 and 4 (N=21, 22), the first size with three
-passes per layer (N=23), and the mirror pass as the last pass (even and odd
-P at two passes per layer)."""
+"""GPU parity of whole circuits and gradients on half states: only the
+amplitudes with qubit N-1 = 0 are swept.  N = 16..19 as one cooperative
+launch (every CTA size, even and odd P), N >= 20 as passes at the edges of
+their tile geometries: rows of 16 amplitudes (N=20), paired rows of 8 and 4
+(N=21, 22), the first size with three passes per layer (N=23), the mirror
+pass as the last pass, and more layers than either keeps tables for."""
 import numpy as np
 import pytest
 
@@ -23,12 +23,13 @@ def graph(kind, n, rng):
     return complete_int(n, rng, -7, 9)
 
 
-@pytest.mark.parametrize("n,P,kind", [(17, 1, "int"), (17, 2, "fp"), (18, 1, "fp"),
+@pytest.mark.parametrize("n,P,kind", [(16, 3, "int"), (16, 2, "wide"), (17, 1, "int"),
+                                      (17, 2, "fp"), (17, 7, "int"), (18, 1, "fp"),
                                       (18, 2, "wide"), (19, 3, "int"), (20, 1, "fp"),
                                       (21, 2, "int"), (22, 1, "int"), (22, 2, "fp"),
                                       (23, 1, "fp"), (23, 2, "int"),
                                       # more layers than the shared layer tables hold
-                                      (17, 66, "fp"), (17, 65, "int")])
+                                      (17, 66, "fp"), (17, 65, "int"), (17, 40, "int")])
 def test_half_state_forward(ctx, oracle, n, P, kind):
     rng = np.random.default_rng(1000 * n + P)
     W = graph(kind, n, rng)
@@ -47,7 +48,9 @@ def test_half_state_forward(ctx, oracle, n, P, kind):
     assert abs(e - eo) <= ENERGY_RTOL * max(1.0, abs(eo), np.abs(W).sum())
 
 
-@pytest.mark.parametrize("n,P,kind", [(17, 1, "fp"), (18, 2, "int"), (17, 3, "wide"),
+@pytest.mark.parametrize("n,P,kind", [(16, 4, "fp"), (17, 1, "fp"), (18, 2, "int"),
+                                      (17, 3, "wide"), (19, 3, "int"), (17, 36, "int"),
+                                      (17, 65, "fp"),
                                       (20, 1, "int"), (21, 2, "fp")])
 def test_half_state_gradient(ctx, oracle, n, P, kind):
     rng = np.random.default_rng(2000 * n + P)
