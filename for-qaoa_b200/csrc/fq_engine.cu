@@ -655,7 +655,7 @@ int fq_qaoa_forward(fq_ctx* ctx, void* sv, int N, int P, const double* graph,
         FQ_CHECK(isfinite(gammas[p]) && isfinite(betas[p]), FQ_ERR_INVALID,
                  "non-finite angle at layer %d", p);
     GraphPrep g;
-    if (N <= kSmallKernelQubits && !mid_ok(ctx, N, P)) {
+    if (N <= kSmallJobMaxQubits) {
         FQ_TRY(prep_graph(graph, N, g));
         FQ_TRY(run_small(ctx, g, P, gammas, betas, SJ_STATE, (double2*)sv, ctx->result));
         return energy ? read_result(ctx, energy) : FQ_OK;

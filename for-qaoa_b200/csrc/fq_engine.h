@@ -85,7 +85,7 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
 int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,
                  double* grad_beta);
 
-// Small instances (fq_small.cuh, N <= kSmallKernelQubits).  small_job fills a
+// Small instances (fq_small.cuh, N <= kSmallJobMaxQubits).  small_job fills a
 // descriptor (its pointers apart) and its small_words(N, P) data words: the
 // weights, then the layers.
 // cap: phase-table entries there is room for; most: entries of one layer's

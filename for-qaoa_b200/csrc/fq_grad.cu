@@ -1,6 +1,6 @@
 // fq_grad.cu -- <C> and its adjoint gradient with respect to every gamma_k
 // and beta_k in one forward and one reverse sweep (fq_qaoa_energy_grad); up
-// to kSmallKernelQubits qubits on chip (fq_small.cuh).
+// to kSmallJobMaxQubits qubits on chip (fq_small.cuh).
 #include <math.h>
 #include <string.h>
 
@@ -66,10 +66,6 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     const std::vector<PassPlan> plan = plan_layer(N, true);
     const int npass = (int)plan.size();
     FQ_CHECK(1 + P + P * npass < kResultWords, FQ_ERR_INVALID, "P=%d too large", P);
-    if (N <= kSmallKernelQubits && !mid_ok(ctx, N, P)) {
-        FQ_TRY(prep_graph(graph, N, g));
-        return run_small(ctx, g, P, gammas, betas, SJ_GRAD, nullptr, ctx->result);
-    }
     if (mid_ok(ctx, N, P)) {
         FQ_TRY(prep_graph(graph, N, g));
         return run_mid(ctx, g, P, gammas, betas, SJ_GRAD, (double2*)sv, (double2*)costate,
@@ -209,7 +205,7 @@ int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,
     const int npass = (int)plan_layer(N, true).size();
     const double* r = ctx->result;
     FQ_TRY(check_device_error(ctx));
-    if (N <= kSmallKernelQubits || mid_ok(ctx, N, P)) {  // run_small's and run_mid's results
+    if (N <= kSmallJobMaxQubits || mid_ok(ctx, N, P)) {  // run_small's and run_mid's results
         *energy = r[0];
         std::copy(r + 1, r + 1 + P, grad_gamma);
         std::copy(r + 1 + P, r + 1 + 2 * P, grad_beta);

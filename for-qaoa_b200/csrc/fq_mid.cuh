@@ -54,6 +54,7 @@ __host__ __device__ constexpr size_t mid_smem_bytes(int nb, bool grad) {
            kMidTable * sizeof(double2);
 }
 static_assert(mid_smem_bytes(kMidMaxBits, true) <= 227 * 1024, "one CTA per SM");
+static_assert((12 * 13 + 16 + (2 * kSumLayers + 1) * kSmallWarps) % 2 == 0, "aligned tables");
 
 // All CTAs of the grid (all resident: cooperative launch).  False if the
 // bounded wait gave up.

@@ -5,8 +5,8 @@
 // a thread of its own, so the ~30 kernel launches of a larger request are
 // issued by its lane's thread, in parallel with the other lanes':
 //   - small instances (N <= 15) are packed into launches of the small-instance
-//     kernels (fq_small.cuh): one CTA each up to 13 qubits, a cluster of
-//     2^(N-13) CTAs above, one launch per size class, side by side on streams
+//     kernels (fq_small.cuh): one CTA each up to 12 qubits, a cluster of
+//     2^(N-12) CTAs above, one launch per size class, side by side on streams
 //     of their own; two batches can be in flight, and a batch takes every
 //     small request queued when it launches (up to its capacity);
 //   - larger instances run on lanes (an fq_ctx each: its own stream and

@@ -46,7 +46,7 @@ namespace {
 // The largest of the one-CTA classes, which share their kernels.
 size_t small_smem_max(bool grad) {
     size_t m = 0;
-    for (int c = 0; c <= 4; c++) m = std::max(m, small_smem_bytes(c, grad, true));
+    for (int c = 0; c <= 3; c++) m = std::max(m, small_smem_bytes(c, grad, true));
     return m;
 }
 
@@ -74,7 +74,7 @@ int launch_cluster(Fn fn, int cb, int njobs, size_t smem, cudaStream_t st, void*
 template <int C, bool GRAD>
 int launch_class(const SmallArgs* one, const SmallJob* jobs, int njobs, cudaStream_t st) {
     void* args[1] = {one ? (void*)one : (void*)&jobs};
-    if constexpr (C <= 4) {
+    if constexpr (C <= 3) {
         const size_t smem = small_smem_bytes(C, GRAD, one != nullptr);
         const void* fn = one ? (const void*)k_small_one<GRAD> : (const void*)k_small_batch<GRAD>;
         // Every class shares the function, and threads set this concurrently:
@@ -87,7 +87,7 @@ int launch_class(const SmallArgs* one, const SmallJob* jobs, int njobs, cudaStre
         FQ_CUDA(cudaLaunchKernel(fn, dim3((unsigned)njobs), dim3(threads), args, smem, st));
         return FQ_OK;
     } else {
-        constexpr int CB = C - 4;
+        constexpr int CB = C - 3;
         const size_t smem = small_cluster_smem_bytes(GRAD);
         const void* fn = one ? (const void*)k_small_cluster_one<CB, GRAD>
                              : (const void*)k_small_cluster_batch<CB, GRAD>;
@@ -105,8 +105,7 @@ int launch_any(int c, const SmallArgs* one, const SmallJob* jobs, int njobs, cud
         case 3: return launch_class<3, GRAD>(one, jobs, njobs, st);
         case 4: return launch_class<4, GRAD>(one, jobs, njobs, st);
         case 5: return launch_class<5, GRAD>(one, jobs, njobs, st);
-        case 6: return launch_class<6, GRAD>(one, jobs, njobs, st);
-        default: return launch_class<7, GRAD>(one, jobs, njobs, st);
+        default: return launch_class<6, GRAD>(one, jobs, njobs, st);
     }
 }
 

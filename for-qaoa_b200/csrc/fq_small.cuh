@@ -1,5 +1,5 @@
-// fq_small.cuh -- whole QAOA instances on chip: up to 13 qubits in one CTA,
-// 14..16 qubits in a cluster of 2, 4 or 8 CTAs.
+// fq_small.cuh -- whole QAOA instances on chip: up to 12 qubits in one CTA,
+// 13..15 qubits in a cluster of 2, 4 or 8 CTAs.
 //
 // An instance keeps psi and, for the gradient, lambda in registers (8
 // amplitudes of each per thread) for the whole circuit; shared memory only
@@ -14,18 +14,20 @@
 // layer, back up.  On the half state RX on the top qubit pairs x with ~x, so
 // the layer's last exchange reads both and combines them.
 //
-// Cluster: CTA `rank` holds a tile of 2^12, alternately the mirror tile
-// (qubits 0..10 and N-1) and the strided tile (qubits 11..N-2, the tile's
-// top bits) of the engine's passes.  As in the engine's fused schedule a
+// Cluster: CTA `rank` holds a tile of 2^11, alternately the mirror tile
+// (qubits 0..9 and N-1) and the strided tile (qubits 10..N-2, the tile's top
+// bits), as in the engine's passes.  As in the engine's fused schedule a
 // layer ends on the tile the next one starts on, so each layer takes one
 // exchange through distributed shared memory.
 //
 // Eight amplitudes per thread and one rolled copy of the rounds.  On B200,
-// kernel times in microseconds: N=12 p=4 gradient (integer weights) 42.6,
-// N=15 p=6 (FP64 weights, 4 CTAs) 156; sixteen per thread 41.8 and 163 (one
-// warp per scheduler waits for its own results where eight pay a third
-// exchange); sixteen with every round unrolled 46 and 143, but 92 and 223
-// with a cold instruction cache, which is a batch's or a first call's case.
+// kernel times in microseconds with tiles of 2^12 per CTA in clusters: N=12
+// p=4 gradient (integer weights) 42.6, N=15 p=6 (FP64 weights) 156; sixteen
+// per thread 41.8 and 163 (one warp per scheduler waits for its own results
+// where eight pay a third exchange); sixteen with every round unrolled 46 and
+// 143, but 92 and 223 with a cold instruction cache, which is a batch's or a
+// first call's case.  Tiles of 2^11 (twice the CTAs) took the N=15 call from
+// 178 to 133.
 //
 // Only the tangent form of the reduced RX is needed: the cotangent gate
 // [[u,-i],[-i,u]] is -i X [[1,iu],[iu,1]], and X on every qubit leaves these
@@ -42,7 +44,7 @@
 // (FP64 pipe half busy), 12 k phases, 6 k set-up; in a cluster the exchange
 // between CTAs adds 4.8 k cycles per layer and direction.  Against the
 // shared-memory butterflies this replaces (whole calls, A/B in one call):
-// gradient N=12 p=4 66 against 258 us, N=15 p=6 179 against 607 us; forward
+// gradient N=12 p=4 64 against 260 us, N=15 p=6 133 against 627 us; forward
 // N=9 p=2 31 against 72 us.
 #pragma once
 
@@ -62,13 +64,16 @@ __host__ __device__ constexpr size_t small_slots(int nb) {
 // weights keep a phase per amplitude in the first vector's buffer instead.
 constexpr int kSmallBits = 3;   // register bits
 constexpr int kSmallRegs = 8;
-constexpr int kSmallThreads = 512;  // of the largest CTA
+constexpr int kSmallThreads = 256;  // of the largest CTA
 constexpr int kSmallWarps = kSmallThreads / 32;
-constexpr int kWsStride = 17;   // row stride of the weights (kSmallKernelQubits rows)
+constexpr int kWsStride = 17;   // row stride of the weights (kSmallJobMaxQubits rows)
 constexpr int kSumLayers = 32;  // layers whose sums are kept before they are written out
+// Doubles of the weights and the sums, an even number (16-byte pieces follow).
 constexpr size_t kSmallFixed =
-    sizeof(double) * (kSmallKernelQubits * kWsStride + (2 * kSumLayers + 1) * kSmallWarps + 2 * kSumLayers + 2);
-// One-CTA classes 0..4 (nb = 8..12).
+    sizeof(double) * ((kSmallJobMaxQubits * kWsStride + (2 * kSumLayers + 1) * kSmallWarps +
+                       2 * kSumLayers + 2) / 2 * 2 + 2);
+static_assert(kSmallFixed % sizeof(double2) == 0 && small_slots(8) % 2 == 0, "aligned tables");
+// One-CTA classes 0..3 (nb = 8..11).
 __host__ __device__ inline size_t small_smem_bytes(int c, bool grad, bool alone) {
     const size_t s = small_slots(8 + c);
     return (grad ? 2 : 1) * s * sizeof(double2) + s * sizeof(double) + kSmallFixed +
@@ -77,13 +82,13 @@ __host__ __device__ inline size_t small_smem_bytes(int c, bool grad, bool alone)
 // Clusters: integer weights keep 4-byte cut values and the phase table in
 // the second half of the cut values' room.
 __host__ __device__ inline size_t small_cluster_smem_bytes(bool grad) {
-    const size_t s = small_slots(12);
+    const size_t s = small_slots(11);
     return (grad ? 2 : 1) * s * sizeof(double2) + 2 * s * sizeof(double) + kSmallFixed;
 }
 
 // Weights into shared memory (symmetric, zero-padded rows), all threads.
 __device__ __forceinline__ void small_weights(const SmallJob& J, double* ws, int nthreads) {
-    for (int i = threadIdx.x; i < kSmallKernelQubits * kWsStride; i += nthreads) ws[i] = 0;
+    for (int i = threadIdx.x; i < kSmallJobMaxQubits * kWsStride; i += nthreads) ws[i] = 0;
     __syncthreads();
     const int N = J.N;
     for (int e = threadIdx.x; e < N * N; e += nthreads) {
@@ -161,7 +166,7 @@ struct SmallLay {
 };
 
 // One instance on one CTA (CB = 0, run-time nb) or on a cluster of 2^CB
-// CTAs (nb = 12).  blockDim.x may exceed the 2^(nb-4) threads that hold
+// CTAs (nb = 11).  blockDim.x may exceed the 2^(nb-4) threads that hold
 // amplitudes: the others help to fill the phase tables.
 template <bool GRAD, int CB>
 struct SmallRun {
@@ -436,7 +441,7 @@ __device__ __forceinline__ void small_run(const SmallJob& J, unsigned char* sm) 
     R.buf = reinterpret_cast<double2*>(sm);
     R.cz = reinterpret_cast<double*>(R.buf + (GRAD ? 2 : 1) * R.S);
     double* ws = R.cz + R.S;
-    R.red = ws + kSmallKernelQubits * kWsStride;
+    R.red = ws + kSmallJobMaxQubits * kWsStride;
     R.tab = R.tab0 = reinterpret_cast<double2*>(ws + kSmallFixed / sizeof(double));
     const int tid = threadIdx.x, N = J.N, P = J.P;
     const bool half = N > nb;
@@ -494,7 +499,7 @@ __device__ __forceinline__ void small_run(const SmallJob& J, unsigned char* sm) 
 }
 
 // One instance, its data behind the descriptor in the kernel parameters.
-constexpr int kSmallArgWords = 120 + 4 * 32;
+constexpr int kSmallArgWords = 105 + 4 * 32;
 struct SmallArgs {
     SmallJob job;
     double data[kSmallArgWords];
@@ -508,14 +513,14 @@ __device__ __forceinline__ SmallJob small_arg_job(const SmallArgs& a) {
 }
 
 template <bool GRAD>
-__global__ void __launch_bounds__(kSmallThreads) k_small_one(const __grid_constant__ SmallArgs a) {
+__global__ void __launch_bounds__(kSmallThreads, 2) k_small_one(const __grid_constant__ SmallArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const SmallJob J = small_arg_job(a);
     small_run<GRAD>(J, smraw);
 }
 
 template <bool GRAD>
-__global__ void __launch_bounds__(kSmallThreads) k_small_batch(const SmallJob* jobs) {
+__global__ void __launch_bounds__(kSmallThreads, 2) k_small_batch(const SmallJob* jobs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const SmallJob J = jobs[blockIdx.x];
     small_run<GRAD>(J, smraw);
@@ -524,7 +529,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_batch(const SmallJob* j
 // ---------------------------------------------------------------- cluster --
 
 // The tile changes hands through distributed shared memory.  Register r of
-// a tile in the top layout (index tid | r << 9) comes from the CTA and slot
+// a tile in the top layout (index tid | r << 8) comes from the CTA and slot
 // that held it as the other kind of tile; which CTA depends on r and, with 8
 // CTAs, on the thread's top bit (the same across a warp, which reads 512
 // contiguous bytes).  The upper half of either tile is the mirror image of
@@ -532,12 +537,12 @@ __global__ void __launch_bounds__(kSmallThreads) k_small_batch(const SmallJob* j
 template <int CB>
 __device__ __forceinline__ void small_fetch(double2 (&v)[kSmallRegs],
                                             double2* const (&peer)[1 << CB], int lo, int hi) {
-    const bool b = threadIdx.x >> 8;
+    const bool b = threadIdx.x >> 7;
 #pragma unroll
     for (int r = 0; r < kSmallRegs; r++) {
-        const int u = r < 4 ? r : 7 - r;  // bits 9, 10 of the unmirrored index
-        // Row bits among the registers (one with 2 CTAs): slots of 2^9.
-        const int row = CB == 1 ? (r & 1) * 544 : 0;
+        const int u = r < 4 ? r : 7 - r;  // bits 8, 9 of the unmirrored index
+        // Row bits among the registers (one with 2 CTAs): slots of 2^8.
+        const int row = CB == 1 ? (r & 1) * 272 : 0;
         const double2* p;
         if (CB == 3)
             p = (r < 4) == b ? peer[(2 * u + 1) & ((1 << CB) - 1)] : peer[(2 * u) & ((1 << CB) - 1)];
@@ -551,17 +556,17 @@ template <int CB, bool GRAD>
 __device__ __forceinline__ void small_cluster_run(const SmallJob& J, unsigned char* sm) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-    constexpr int N = 13 + CB, S = kXTile, l = 11 - CB;
+    constexpr int N = 12 + CB, S = (int)small_slots(11), l = 10 - CB;
     SmallRun<GRAD, CB> R(J);
-    R.nb = 12;
+    R.nb = 11;
     R.nt = kSmallThreads;
-    R.nq = 12;
+    R.nq = 11;
     R.S = S;
     R.on = true;
     R.buf = reinterpret_cast<double2*>(sm);
     double* const cA = reinterpret_cast<double*>(R.buf + (GRAD ? 2 : 1) * S);
     double* const ws = cA + 2 * S;
-    R.red = ws + kSmallKernelQubits * kWsStride;
+    R.red = ws + kSmallJobMaxQubits * kWsStride;
     double* const part = R.red + (2 * kSumLayers + 1) * kSmallWarps;  // read by rank 0
     double* const cB = J.ntab ? cA + S / 2 : cA + S;
     R.tab = R.tab0 = reinterpret_cast<double2*>(cA + S);
@@ -572,16 +577,16 @@ __device__ __forceinline__ void small_cluster_run(const SmallJob& J, unsigned ch
 #pragma unroll
     for (int r = 0; r < (1 << CB); r++) peer[r] = cl.map_shared_rank(R.buf, r);
     small_weights(J, ws, kSmallThreads);
-    // Mirror tile: registers = qubits 9, 10, N-1, the rank's bits from 11;
-    // strided tile: registers = tile bits 9..11 (and tile bit 8 of the thread
-    // is qubit 11 with 8 CTAs), the rank's bits from l.
-    auto q = [](int j) { return j < l ? j : j + 11 - l; };
-    const int zB = CB == 3 ? (tid & 255) | ((tid >> 8) << q(8)) : tid;
-    R.template put_cuts<N>(ws, cA, tid | (rank << 11), 9, 10, N - 1);
-    R.template put_cuts<N>(ws, cB, zB | (rank << l), q(9), q(10), q(11));
+    // Mirror tile: registers = qubits 8, 9, N-1, the rank's bits from 10;
+    // strided tile: registers = tile bits 8..10 (and tile bit 7 of the thread
+    // is qubit 10 with 8 CTAs), the rank's bits from l.
+    auto q = [](int j) { return j < l ? j : j + 10 - l; };
+    const int zB = CB == 3 ? (tid & 127) | ((tid >> 7) << q(7)) : tid;
+    R.template put_cuts<N>(ws, cA, tid | (rank << 10), 8, 9, N - 1);
+    R.template put_cuts<N>(ws, cB, zB | (rank << l), q(8), q(9), q(10));
     const int row = tid & ((1 << l) - 1);  // the row bits (all of tid but with 8 CTAs)
     const int lo = pslot(row | (rank << l));
-    const int hiB = pslot(2048 | (2047 - (row | (rank << l))));
+    const int hiB = pslot(1024 | (1023 - (row | (rank << l))));
     const int hiA = pslot(((1 << l) - 1 - row) | (((2 << CB) - 1 - rank) << l));
     // The tile leaves from layout L; the other kind of tile arrives in H.  The
     // barrier_wait that matches the arrive comes before buf is written again.
@@ -632,10 +637,10 @@ __device__ __forceinline__ void small_cluster_run(const SmallJob& J, unsigned ch
             const int i = (tid & lom) | ((tid & ~lom) << kSmallBits) | (r << p);
             int x;
             if (strided) {
-                x = (i & ((1 << l) - 1)) | (rank << l) | ((i >> l) << 11);
+                x = (i & ((1 << l) - 1)) | (rank << l) | ((i >> l) << 10);
             } else {
-                x = (i & 2047) | (rank << 11);
-                if (i >> 11) x = M - x;
+                x = (i & 1023) | (rank << 10);
+                if (i >> 10) x = M - x;
             }
             const double2 a = small_turned(R.v[r], J.rot);
             J.state[x] = a;
@@ -689,7 +694,7 @@ __device__ __forceinline__ void small_cluster_run(const SmallJob& J, unsigned ch
 }
 
 template <int CB, bool GRAD>
-__global__ void __launch_bounds__(kSmallThreads)
+__global__ void __launch_bounds__(kSmallThreads, 2)
     k_small_cluster_one(const __grid_constant__ SmallArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const SmallJob J = small_arg_job(a);
@@ -697,7 +702,7 @@ __global__ void __launch_bounds__(kSmallThreads)
 }
 
 template <int CB, bool GRAD>
-__global__ void __launch_bounds__(kSmallThreads) k_small_cluster_batch(const SmallJob* jobs) {
+__global__ void __launch_bounds__(kSmallThreads, 2) k_small_cluster_batch(const SmallJob* jobs) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const SmallJob J = jobs[blockIdx.x >> CB];
     small_cluster_run<CB, GRAD>(J, smraw);

@@ -1,6 +1,6 @@
 // fq_small.h -- job descriptor of the small-instance kernels (fq_small.cuh):
-// one whole QAOA instance per CTA (N <= 13) or per cluster of 2^(N-13) CTAs
-// (N = 14..16).
+// one whole QAOA instance per CTA (N <= 12) or per cluster of 2^(N-12) CTAs
+// (N = 13..15).
 #pragma once
 
 #include <vector>
@@ -9,9 +9,9 @@
 
 namespace fq {
 
-constexpr int kSmallMaxQubits = 13;     // qubits of a one-CTA instance
-constexpr int kSmallJobMaxQubits = 15;  // qubits of a request that needs no buffers (FQ_SMALL_MAX_QUBITS)
-constexpr int kSmallKernelQubits = 16;  // qubits of the largest instance a cluster holds
+constexpr int kSmallMaxQubits = 12;     // qubits of a one-CTA instance
+constexpr int kSmallJobMaxQubits = 15;  // of a cluster's, and of a request that needs no
+                                        // buffers (FQ_SMALL_MAX_QUBITS)
 
 enum { SJ_GRAD = 1, SJ_STATE = 2 };
 
@@ -31,20 +31,16 @@ struct SmallJob {
 // Data words of a job behind its descriptor.
 __host__ __device__ inline int small_words(int N, int P) { return N * (N - 1) / 2 + 4 * P; }
 
-// Size class of an N-qubit instance: 0..4 for one CTA of 2^(8..12)
-// amplitudes (a half state from N = 9 on), 5..7 for clusters of 2, 4, 8.
-constexpr int kSmallClasses = 8;
-__host__ __device__ inline int small_class(int N) {
-    return N <= 9 ? 0 : N <= kSmallMaxQubits ? N - 9 : N - kSmallMaxQubits + 4;
-}
+// Size class of an N-qubit instance: 0..3 for one CTA of 2^(8..11)
+// amplitudes (a half state from N = 9 on), 4..6 for clusters of 2, 4, 8.
+constexpr int kSmallClasses = 7;
+__host__ __device__ inline int small_class(int N) { return N <= 9 ? 0 : N - 9; }
 // Phase-table entries of a job of size class c: what is left of the shared
-// memory at the residency its registers allow in a batch (4 CTAs per SM and
-// more up to class 2, two of class 3, one of class 4), and more for an
-// instance alone.  Clusters use the room integer cut values leave free.
+// memory at the residency its registers allow in a batch (two CTAs per SM of
+// class 3, more below), and more for an instance alone.  Clusters use the
+// room integer cut values leave free.
 __host__ __device__ inline int small_table_cap(int c, bool alone) {
-    if (c > 4) return 2048;
-    if (c == 4) return 2816;
-    return alone ? 4096 : 128 << c;
+    return c > 3 ? 1088 : alone ? 4096 : 128 << c;
 }
 
 // A table is worth its sincos (half its entries) up to the 2^(N-1) amplitudes.

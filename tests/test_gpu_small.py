@@ -1,5 +1,5 @@
-"""GPU parity of instances held on chip (N <= 16: one CTA up to 13 qubits, a
-cluster of 2, 4 or 8 CTAs above) at the edges of their layouts: states
+"""GPU parity of instances held on chip (one CTA up to 12 qubits, a
+cluster of 2, 4 or 8 CTAs up to 15) at the edges of their layouts: states
 smaller than the smallest CTA, whole and half states, every CTA and cluster
 size, phase tables kept for all layers, refilled per layer and absent, and
 circuits deeper than the kernel parameters and the sum groups hold."""
