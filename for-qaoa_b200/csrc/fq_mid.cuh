@@ -45,15 +45,16 @@ struct MidArgs {
 };
 static_assert(sizeof(MidArgs) <= 4096, "kernel parameters");
 
-constexpr int kMidTable = 4096;  // phase-table entries
-__host__ __device__ constexpr size_t mid_smem_bytes(int nb, bool grad) {
+constexpr int kMidTable = 4096;  // phase-table entries at most
+// `table`: entries of the job's phase tables.
+__host__ __device__ constexpr size_t mid_smem_bytes(int nb, bool grad, int table) {
     return (grad ? 2 : 1) * small_slots(nb) * sizeof(double2) +
            2 * small_slots(nb) * sizeof(double) +
            sizeof(double) * ((kMidMaxQubits * kMidStride + 1) / 2 * 2 + 12 * 13 + 16 +
                              (2 * kSumLayers + 1) * kSmallWarps) +
-           kMidTable * sizeof(double2);
+           table * sizeof(double2);
 }
-static_assert(mid_smem_bytes(kMidMaxBits, true) <= 227 * 1024, "one CTA per SM");
+static_assert(mid_smem_bytes(kMidMaxBits, true, kMidTable) <= 227 * 1024, "one CTA per SM");
 static_assert((12 * 13 + 16 + (2 * kSumLayers + 1) * kSmallWarps) % 2 == 0, "aligned tables");
 
 // All CTAs of the grid (all resident: cooperative launch).  False if the

@@ -81,6 +81,7 @@ struct Lane {
 
 constexpr int kBatchCap = 4096;           // small instances per launch
 constexpr int kExpressN = 20;             // lane requests up to this size go first
+constexpr double kSpinS = 0.0005;         // polled without sleeping (see lane_loop)
 constexpr double kEvictIdleS = 0.05;      // a session idle this long may lose its buffers
 constexpr int kHeavyN = 24;               // requests this large fill the GPU on their own
 
@@ -423,6 +424,7 @@ struct fq_server {
                 cv_lane.notify_all();
                 continue;
             }
+            const double t0 = now_s();
             while (true) {
                 const cudaError_t q = cudaEventQuery(L.done);
                 if (q == cudaSuccess) break;
@@ -430,7 +432,13 @@ struct fq_server {
                     cudaGetLastError();
                     break;  // grad_collect reports the failure
                 }
-                std::this_thread::sleep_for(std::chrono::microseconds(20));
+                // A 20 us sleep takes 70 or more, as long as a request of up to
+                // 20 qubits: those are polled (yielding) for their first half
+                // millisecond.
+                if (L.cur.N <= kExpressN && now_s() - t0 < kSpinS)
+                    std::this_thread::yield();
+                else
+                    std::this_thread::sleep_for(std::chrono::microseconds(20));
             }
             complete_large(L);
             cv_lane.notify_all();  // the session may have a next step queued
@@ -440,6 +448,7 @@ struct fq_server {
     // ---- scheduler loop -----------------------------------------------------
     void loop() {
         cudaSetDevice(device);
+        double t_work = 0;
         while (true) {
             bool worked = false, pending = false;
             for (auto& B : batches) {
@@ -461,12 +470,18 @@ struct fq_server {
                 }
                 pending |= B.busy;
             }
-            if (worked) continue;
+            if (worked) {
+                t_work = now_s();
+                continue;
+            }
             std::unique_lock<std::mutex> lk(mu);
             if (stop && small_q.empty() && !pending) break;
             if (pending) {
-                lk.unlock();
-                std::this_thread::sleep_for(std::chrono::microseconds(10));
+                lk.unlock();  // a batch in flight: as in lane_loop
+                if (now_s() - t_work < kSpinS)
+                    std::this_thread::yield();
+                else
+                    std::this_thread::sleep_for(std::chrono::microseconds(10));
             } else {
                 cv_work.wait_for(lk, std::chrono::milliseconds(5));
             }

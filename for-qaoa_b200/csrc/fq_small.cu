@@ -145,10 +145,11 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
     }
     a.base = ctx->counter_base;
     const void* fn = grad ? (const void*)k_mid<true> : (const void*)k_mid<false>;
-    const size_t smem = mid_smem_bytes(nb, grad);
+    // Only the tables the job has: instances of other lanes fit beside it.
+    const size_t smem = mid_smem_bytes(nb, grad, a.job.ntab * (a.job.keep ? P : 1));
     // The largest size for every N: contexts on other threads set it too.
     FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)mid_smem_bytes(kMidMaxBits, grad)));
+                                 (int)mid_smem_bytes(kMidMaxBits, grad, kMidTable)));
     void* args[1] = {&a};
     const int tok = prof_begin(ctx);
     FQ_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem,
