@@ -27,9 +27,8 @@ struct fq_ctx {
     size_t tcut_bytes = 0;
     long long tcut_version = -1;  // g_version the tables were built for (-1: none)
     int tcut_n = -1;              // and N
-    unsigned* d_counter = nullptr;   // grid barrier of k_mid: arrivals since its last reset,
-    unsigned counter_base = 0;       // expected when the next launch starts,
-    bool counter_lost = false;       // unknown after a wait that gave up
+    unsigned* d_counter = nullptr;   // grid barrier of k_mid: arrivals so far
+    bool counter_lost = false;       // not known to be between two launches' (see run_mid)
     bool cooperative = false;        // the device takes cooperative launches
     unsigned char* d_img = nullptr;  // static cut tables of the plan's geometries, built with them
     int partial_cap = 0;

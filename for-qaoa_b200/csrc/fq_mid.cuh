@@ -37,14 +37,14 @@ struct MidArgs {
     SmallJob job;      // state = psi's buffer (a whole state with SJ_STATE)
     double2* lam;      // lambda's buffer (SJ_GRAD)
     double* partial;   // (2P + 1) x CTAs
-    unsigned* counter; // grid barrier: arrivals since the last reset
+    unsigned* counter; // grid barrier: arrivals, a multiple of kMidMaxCtas between launches
     int nb;
-    unsigned base;     // its value at the start of this launch
     int* err;
     double data[kMidWords];
 };
 static_assert(sizeof(MidArgs) <= 4096, "kernel parameters");
 
+constexpr int kMidMaxCtas = 128;
 constexpr int kMidTable = 4096;  // phase-table entries at most
 // `table`: entries of the job's phase tables.
 __host__ __device__ constexpr size_t mid_smem_bytes(int nb, bool grad, int table) {
@@ -204,7 +204,11 @@ __global__ void __launch_bounds__(1 << (kMidMaxBits - kSmallBits)) k_mid(const _
         const int x = (rank << h) | (i & lowm);
         return i >> h ? M - x : x;
     };
-    unsigned target = a.base;
+    // The barrier counts up without a reset, so that a captured launch can be
+    // replayed: every launch finds and leaves a multiple of kMidMaxCtas, and
+    // fewer than that many CTAs can have arrived before this one has.
+    unsigned target = 0;
+    if (tid == 0) target = *(volatile unsigned*)a.counter & ~(unsigned)(kMidMaxCtas - 1);
     // The tile (in the top layout) for this CTA's tile of the other kind.
     auto change = [&](bool strided, bool dual) -> bool {
 #pragma unroll
@@ -289,6 +293,10 @@ __global__ void __launch_bounds__(1 << (kMidMaxBits - kSmallBits)) k_mid(const _
     const int nv = GRAD ? 2 * P : 0;
     if (tid == 0) a.partial[nv * grid + rank] = R.row_sum(2 * kSumLayers);
     if (!mid_barrier(a, target += grid)) return;
+    if (rank == 0 && tid == 0) {
+        const unsigned pad = (0u - target) & (kMidMaxCtas - 1);
+        if (pad) atomicAdd(a.counter, pad);
+    }
     // Value v's partial sums, in a fixed order, on a warp of CTA v % grid.
     for (int i = rank; i <= nv; i += grid) {
         if ((i / grid) % (R.nt / 32) != tid >> 5) continue;

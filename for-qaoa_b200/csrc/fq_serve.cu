@@ -52,8 +52,7 @@ size_t session_bytes(int N) { return 2 * (sizeof(double2) << N); }
 struct Req {
     uint64_t ticket = 0, session = 0;
     int N = 0, P = 0;
-    SmallJob job;               // small instances: descriptor and data words
-    std::vector<double> data;
+    GraphPrep prep;             // small instances (the scheduler thread fills their jobs)
     std::vector<double> graph;  // N*N upper triangle (large instances)
     std::vector<double> gammas, betas;
     double t_submit = 0, t_start = 0;
@@ -134,6 +133,7 @@ struct fq_server {
     cudaStream_t side[kSmallClasses] = {};  // of both batches
     std::map<uint64_t, Session> sessions;  // guarded by mu
     std::deque<Req> small_q, large_q;      // guarded by mu
+    std::deque<Req> small_local;           // the scheduler's own: taken, not yet launched
     std::vector<fq_result> done;           // guarded by mu
     std::mutex mu;
     std::condition_variable cv_done, cv_work, cv_lane;
@@ -143,6 +143,7 @@ struct fq_server {
     long long in_flight = 0;
     // Written by the worker, read by fq_server_stats.
     std::atomic<long long> launches{0}, batched{0}, laned{0};
+    std::atomic<int> small_waiting{0};  // small_q's size, for a look without the lock
     int error = FQ_OK;
     char errmsg[256] = "";
 
@@ -155,8 +156,8 @@ struct fq_server {
         }
     }
 
-    void finish(const Req& r, int status, const double* e, const double* gg, const double* gb,
-                double t_start) {
+    static fq_result result_of(const Req& r, int status, const double* e, const double* gg,
+                               const double* gb, double t_start) {
         fq_result o;
         memset(&o, 0, sizeof(o));
         o.ticket = r.ticket;
@@ -174,6 +175,12 @@ struct fq_server {
         o.t_submit = r.t_submit;
         o.t_start = t_start;
         o.t_done = now_s();
+        return o;
+    }
+
+    void finish(const Req& r, int status, const double* e, const double* gg, const double* gb,
+                double t_start) {
+        const fq_result o = result_of(r, status, e, gg, gb, t_start);
         std::lock_guard<std::mutex> lk(mu);
         done.push_back(o);
         in_flight--;
@@ -182,7 +189,7 @@ struct fq_server {
 
     // ---- small instances (one CTA each, or one cluster of CTAs) --------------
     static size_t job_bytes(const Req& r) {
-        return sizeof(SmallJob) + sizeof(double) * r.data.size();
+        return sizeof(SmallJob) + sizeof(double) * small_words(r.N, r.P);
     }
 
     int launch_batch(Batch& B) {
@@ -201,11 +208,12 @@ struct fq_server {
         B.out_off.assign(nj, 0);
         for (int i = 0; i < nj; i++) {
             const Req& r = B.reqs[i];
-            SmallJob d = r.job;
-            memcpy(hd + off, r.data.data(), sizeof(double) * r.data.size());
+            SmallJob d;
+            small_job(r.prep, r.P, r.gammas.data(), r.betas.data(), SJ_GRAD,
+                      small_table_cap(small_class(r.N), false), small_table_most(r.N), d, hd + off);
             d.w = dd + off;
             d.lay = d.w + r.N * (r.N - 1) / 2;
-            off += r.data.size();
+            off += small_words(r.N, r.P);
             d.out = B.out + o;
             B.out_off[i] = o;
             o += 1 + 2 * r.P;
@@ -244,28 +252,47 @@ struct fq_server {
         return FQ_OK;
     }
 
+    // All of a batch's results under one lock: the clients submit meanwhile.
     void complete_batch(Batch& B) {
+        std::vector<fq_result> res;
+        res.reserve(B.reqs.size());
         for (size_t i = 0; i < B.reqs.size(); i++) {
             const Req& r = B.reqs[i];
             const double* out = B.out + B.out_off[i];
-            finish(r, FQ_OK, out, out + 1, out + 1 + r.P, B.t_start);
+            res.push_back(result_of(r, FQ_OK, out, out + 1, out + 1 + r.P, B.t_start));
         }
         B.reqs.clear();
         B.busy = false;
+        std::lock_guard<std::mutex> lk(mu);
+        done.insert(done.end(), res.begin(), res.end());
+        in_flight -= (long long)res.size();
+        cv_done.notify_all();
     }
 
-    // Takes queued small requests that fit one launch (in order).
+    // Takes queued small requests that fit one launch (in order).  The queue
+    // changes hands whole, so the lock clients submit under is held for a
+    // moment only.
     void take_small(Batch& B) {
+        if (small_waiting.load() > 0) {
+            std::lock_guard<std::mutex> lk(mu);
+            if (small_local.empty())
+                small_local.swap(small_q);
+            else
+                while (!small_q.empty()) {
+                    small_local.push_back(std::move(small_q.front()));
+                    small_q.pop_front();
+                }
+            small_waiting = 0;
+        }
         size_t bytes = 0;
         int outw = 0;
-        std::lock_guard<std::mutex> lk(mu);
-        while (!small_q.empty() && (int)B.reqs.size() < kBatchCap) {
-            const Req& r = small_q.front();
+        while (!small_local.empty() && (int)B.reqs.size() < kBatchCap) {
+            const Req& r = small_local.front();
             if (bytes + job_bytes(r) > kBatchBytes || outw + 1 + 2 * r.P > kBatchOut) break;
             bytes += job_bytes(r);
             outw += 1 + 2 * r.P;
-            B.reqs.push_back(std::move(small_q.front()));
-            small_q.pop_front();
+            B.reqs.push_back(std::move(small_local.front()));
+            small_local.pop_front();
         }
     }
 
@@ -474,17 +501,17 @@ struct fq_server {
                 t_work = now_s();
                 continue;
             }
-            std::unique_lock<std::mutex> lk(mu);
-            if (stop && small_q.empty() && !pending) break;
-            if (pending) {
-                lk.unlock();  // a batch in flight: as in lane_loop
+            if (pending) {  // a batch in flight: as in lane_loop
                 if (now_s() - t_work < kSpinS)
                     std::this_thread::yield();
                 else
                     std::this_thread::sleep_for(std::chrono::microseconds(10));
-            } else {
-                cv_work.wait_for(lk, std::chrono::milliseconds(5));
+                continue;
             }
+            std::unique_lock<std::mutex> lk(mu);
+            if (!small_q.empty() || !small_local.empty()) continue;
+            if (stop) break;
+            cv_work.wait_for(lk, std::chrono::milliseconds(5));
         }
     }
 };
@@ -630,9 +657,7 @@ int fq_server_submit(fq_server* S, const fq_request* q, uint64_t* ticket) {
     r.betas.assign(q->betas, q->betas + q->P);
     const bool small = q->N <= kSmallJobMaxQubits;
     if (small) {
-        r.data.resize(small_words(q->N, q->P));
-        small_job(g, q->P, q->gammas, q->betas, SJ_GRAD, small_table_cap(small_class(q->N), false),
-                  small_table_most(q->N), r.job, r.data.data());
+        r.prep = std::move(g);
     } else {
         r.graph.assign(q->graph_upper, q->graph_upper + (size_t)q->N * q->N);
     }
@@ -645,9 +670,10 @@ int fq_server_submit(fq_server* S, const fq_request* q, uint64_t* ticket) {
     r.ticket = S->next_ticket++;
     *ticket = r.ticket;
     S->in_flight++;
-    if (small)
+    if (small) {
         S->small_q.push_back(std::move(r));
-    else {
+        S->small_waiting++;
+    } else {
         Session& ss = S->sessions[r.session];
         ss.queued++;
         ss.closed = false;  // new work reopens a closed session

@@ -122,7 +122,7 @@ static int mid_bits(int N) { return std::max(kMidMinBits, N - 8); }
 
 bool mid_ok(const fq_ctx* ctx, int N, int P) {
     return N >= kMidMinQubits && N <= kMidMaxQubits && P <= kMidMaxLayers &&
-           1 << (N - 1 - mid_bits(N)) <= ctx->num_sms && ctx->cooperative;
+           1 << (N - 1 - mid_bits(N)) <= std::min(ctx->num_sms, kMidMaxCtas) && ctx->cooperative;
 }
 
 int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
@@ -140,10 +140,8 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
     a.err = ctx->err;
     if (ctx->counter_lost) {  // a barrier gave up: its arrivals are not all counted
         FQ_CUDA(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
-        ctx->counter_base = 0;
         ctx->counter_lost = false;
     }
-    a.base = ctx->counter_base;
     const void* fn = grad ? (const void*)k_mid<true> : (const void*)k_mid<false>;
     // Only the tables the job has: instances of other lanes fit beside it.
     const size_t smem = mid_smem_bytes(nb, grad, a.job.ntab * (a.job.keep ? P : 1));
@@ -155,7 +153,6 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
     FQ_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem,
                                         ctx->stream));
     prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
-    ctx->counter_base += (unsigned)(((grad ? 2 : 1) * P + 1) * grid);  // its barriers
     ctx->launches++;
     return FQ_OK;
 }

@@ -64,3 +64,30 @@ def test_half_state_gradient(ctx, oracle, n, P, kind):
     assert abs(e - eo) <= ENERGY_RTOL * max(1.0, abs(eo), np.abs(W).sum())
     assert np.abs(gg - go).max() <= GRAD_TOL * scale
     assert np.abs(gb - bo).max() <= GRAD_TOL * scale
+
+
+@pytest.mark.parametrize("n", [12, 14, 17, 18])
+def test_captured_circuit_replays(fq, oracle, n):
+    """A circuit captured in a CUDA graph gives the same state at every
+    replay (the grid barrier of one launch leaves itself ready for the next)."""
+    import torch
+    rng = np.random.default_rng(n)
+    W = complete_int(n, rng)
+    g, b = angles(rng, 3)
+    want = oracle.qaoa_logical(W, g, b)
+    stream = torch.cuda.Stream()
+    with fq.Context(0, stream.cuda_stream) as c:
+        st = c.state(n)
+        try:
+            c.qaoa_forward(st, W, g, b)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                c.qaoa_forward(st, W, g, b, energy=False)
+            for _ in range(3):
+                st.init_basis0()
+                c.synchronize()
+                graph.replay()
+                torch.cuda.synchronize()
+                assert_state_close(st.to_host(), want, what=f"N={n}")
+        finally:
+            st.free()
