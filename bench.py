@@ -247,15 +247,15 @@ def is_headline(args):
     return args.n == 30 and args.p == 5
 
 
-# The kernels behind each pass kind of the engine at N=30 (tiles of 4096
-# amplitudes; strided tiles of 128-byte rows run paired, 512 threads).
+# The kernels behind each pass kind of the engine at N=30 (half states; tiles
+# of 4096 amplitudes; strided tiles have 128-byte rows).
 KIND_KERNELS = {
     "init_pass": "fq::k_pass, PH_INIT (layer 0: launch-control init + phase + RX, write-only, "
                  "strided tile, paired)",
-    "phase_pass": "fq::k_pass with GM2 (fused two-layer pass: RX, next layer's phase, RX; "
-                  "strided tiles, paired)",
-    "mixer_pass": "fq::k_pass, PH_NONE (RX only: the contiguous pass over qubits 0..11, and "
-                  "the circuit's last pass)",
+    "phase_pass": "fq::k_pass_col (fused two-layer pass: RX, next layer's phase, RX; strided "
+                  "tiles)",
+    "mixer_pass": "fq::k_pass, PH_NONE (RX only: the mirror pass over qubits 0..10 and 29, the "
+                  "last layer's strided pass)",
 }
 
 
@@ -489,7 +489,7 @@ def run_ours(args):
                 "per_layer": {"gbs": layer_gbs, "frac": layer_gbs / peak if layer_gbs else None,
                               "launches": tot_n,
                               "kernels": "every tile pass of the circuit (fq::k_pass, "
-                                         "fq::k_pass_tma)",
+                                         "fq::k_pass_col)",
                               "sweeps_per_layer": tot_n / (args.steps * args.p),
                               "alg_bytes_per_layer": tot_b / (args.steps * args.p),
                               "share_of_step": (tot_ms / ms) if ms else None},
