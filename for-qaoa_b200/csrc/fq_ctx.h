@@ -49,6 +49,7 @@ struct fq_ctx {
         double bytes;
     };
     bool profiling = false;
+    bool chain = true;  // short passes may be launched in chains (chain_pass)
     std::vector<ProfRec> prof_pending;
     std::vector<cudaEvent_t> prof_pool;
     double prof_ms[FQ_KIND_COUNT] = {};

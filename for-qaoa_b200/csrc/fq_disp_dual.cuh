@@ -22,8 +22,8 @@ inline int dual_launch(fq_ctx* ctx, const PassArgs& A, double* gb, double* gg, d
                                  (int)dual_smem_bytes<WT>(kMaxQubits)));
     const i64 grid = std::min<i64>(A.ntiles, (i64)ctx->num_sms);
     const int tok = prof_begin(ctx);
-    fn<<<(unsigned)grid, kPassThreads, dual_smem_bytes<WT>(A.N), ctx->stream>>>(A, gb, gg, gb2);
-    FQ_CUDA(cudaGetLastError());
+    FQ_CUDA(launch_pass(fn, grid, kPassThreads, dual_smem_bytes<WT>(A.N), ctx->stream,
+                        A.chained > 1, A, gb, gg, gb2));
     // The turnaround reads one vector and writes two; ST = false reads two.
     prof_end(ctx, tok, FQ_KIND_ADJOINT, (TURN ? 48.0 : ST ? 64.0 : 32.0) * (double)A.ntiles * kTile);
     ctx->launches++;

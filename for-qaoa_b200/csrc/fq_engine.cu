@@ -527,6 +527,22 @@ bool fuse_enabled() {
 // in one call), N=28 8.73-8.97 against 8.85-8.97, smaller ones within 1%.
 static int last_order(int npass, int j) { return npass == 3 && j > 0 ? 3 - j : j; }
 
+// Whether a pass of ntiles tiles is launched in a chain (0: no, 1: as its
+// first pass, 2: after another pass; PassArgs::chained).  Passes of a few
+// tiles per SM spend a good part of their time on launch, set-up and the last
+// wave.  Whole calls with five layers, one by one against chained:
+//   forward, integer weights   N=20 84.2 / 76.2 us, N=21 106 / 95.2, N=22 166 / 158
+//   forward, FP64 weights      N=20 89.9 / 81.3 us, N=22 175 / 168, N=23 336 / 347
+//   gradient, integer weights  N=20 188 / 175 us, N=21 289 / 275, N=23 984 / 1004
+//   gradient, FP64 weights     N=21 298 / 290 us, N=22 546 / 548, N=23 1045 / 1075
+// hence forward passes up to 4 tiles per SM (N = 22), adjoint passes, whose
+// CTAs have an SM each, up to 2 (N = 21).  Kernels that are timed one by one
+// (profiling), and those of a server's lanes, are launched one by one.
+int chain_pass(const fq_ctx* ctx, i64 ntiles, int per_sm, bool first) {
+    if (!ctx->chain || ctx->profiling || ntiles > (i64)per_sm * ctx->num_sms) return 0;
+    return first ? 1 : 2;
+}
+
 static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g,
                                 const double* gammas, const double* betas, double* energy,
                                 const std::vector<PassPlan>& plan,
@@ -560,6 +576,7 @@ static int engine_forward_fused(fq_ctx* ctx, void* sv, int N, int P, const Graph
             PassArgs A = engine_args(ctx, sv, N, g, plan[idx]);
             A.tcut = tcut[idx];
             A.gx = gx[p];
+            A.chained = chain_pass(ctx, A.ntiles, 4, p == 0 && j == 0);
             const bool last_of_layer = j == npass - 1;
             int ph = PH_NONE;
             if (p == 0 && j == 0) {  // launch-control init + layer-0 phase + RX

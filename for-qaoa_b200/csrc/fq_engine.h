@@ -76,6 +76,7 @@ int engine_forward(fq_ctx* ctx, void* sv, int N, int P, const GraphPrep& g, cons
 // index of the last pass it runs.
 bool engine_fused(const GraphPrep& g, int P);
 int engine_last_pass(const GraphPrep& g, int N, int P);
+int chain_pass(const fq_ctx* ctx, i64 ntiles, int per_sm, bool first);
 
 // The gradient of more than kSmallJobMaxQubits qubits split for asynchronous use: grad_enqueue puts every
 // kernel and the final device-to-host copy of the results on ctx's stream;

@@ -132,6 +132,10 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
         A.sv2 = (double2*)costate;
         const int nt = __builtin_popcount(plan[i].tmask);
         A.gx = gx[k];
+        // Between two passes that do not follow one another directly (sums or
+        // phase tables in between) the chain starts again.
+        A.chained = chain_pass(ctx, A.ntiles, 2,
+                               q == 0 || !batched || (g.integer && !all_tables));
         A.f2 = f[k] * f[k];
         A.sc0 = pow(f[k] * f[k], rotated[k]);
         rotated[k] += nt;

@@ -46,17 +46,43 @@ inline double pass_bytes(const PassArgs& A) {
 // against 242 ms per N=32 circuit (p=3), A/B in one call.
 inline bool pair_ok(const PassArgs& A) { return A.l >= 1 && A.l <= 3 && A.a > A.l && A.ntiles >= 2; }
 
+constexpr size_t kSoloSmem = 120 * 1024;  // more than half an SM's shared memory
+
+// Launch of a pass; chained: it may start before the kernel before it on the
+// stream is complete, and waits in pass_chain.
+template <typename... P, typename... T>
+inline cudaError_t launch_pass(void (*fn)(P...), i64 grid, int threads, size_t smem,
+                               cudaStream_t stream, bool chained, const T&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
 template <typename WT, int PH, int GM, int EX, int ST, int SC, int GM2 = GM_NONE,
           bool PAIR = false, bool MIR = false>
 inline int launch_ldg_as(fq_ctx* ctx, const PassArgs& A) {
     auto fn = k_pass<WT, PH, GM, EX, ST, SC, GM2, PAIR, MIR>;
-    const size_t smem = pass_smem_bytes<WT>(A.N, PAIR);
-    FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    size_t smem = pass_smem_bytes<WT>(A.N, PAIR);
+    // One limit for all launches of this kernel: threads on other contexts may
+    // set it between this line and the launch.
+    const size_t most = std::max<size_t>(smem, kSoloSmem);
+    FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     const i64 units = PAIR ? A.ntiles / 2 : A.ntiles;
+    // One CTA per SM, or the next pass's early CTAs would double up on the SMs
+    // that this one leaves idle and run at half their speed.
+    if (A.chained && units <= ctx->num_sms) smem = most;
     const i64 grid = std::min<i64>(units, (i64)(PAIR ? 1 : ctx->ctas_per_sm) * ctx->num_sms);
     const int tok = prof_begin(ctx);
-    fn<<<(unsigned)grid, PAIR ? 2 * kPassThreads : kPassThreads, smem, ctx->stream>>>(A);
-    FQ_CUDA(cudaGetLastError());
+    FQ_CUDA(launch_pass(fn, grid, PAIR ? 2 * kPassThreads : kPassThreads, smem, ctx->stream,
+                        A.chained > 1, A));
     ctx->last_grid = (int)grid;
     prof_end(ctx, tok, pass_kind<PH, GM, EX, ST>(), pass_bytes<PH, EX, ST>(A));
     ctx->launches++;
@@ -154,8 +180,8 @@ inline int launch_tma(fq_ctx* ctx, const PassArgs& A, const CUtensorMap& map, Tm
     auto fn = k_pass_tma<WT, PH, GM, EX, ST, SC>;
     FQ_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)tma_pass_smem_bytes<WT>(kMaxQubits)));
-    fn<<<(unsigned)grid, kPassThreads, tma_pass_smem_bytes<WT>(A.N), ctx->stream>>>(A, map, G);
-    FQ_CUDA(cudaGetLastError());
+    FQ_CUDA(launch_pass(fn, grid, kPassThreads, tma_pass_smem_bytes<WT>(A.N), ctx->stream,
+                        A.chained > 1, A, map, G));
     ctx->last_grid = (int)grid;
     prof_end(ctx, tok, pass_kind<PH, GM, EX, ST>(), pass_bytes<PH, EX, ST>(A));
     ctx->launches++;

@@ -17,7 +17,8 @@
 // Measured on B200 (whole calls, p=6, in one run; as passes / here): forward
 // N=16 101 / 71 us, N=18 87 / 71, N=19 88 / 79, N=20 93 / 101; gradient N=16
 // 197 / 105, N=18 204 / 120, N=19 206 / 148, N=20 218 / 212: the line lies at
-// N = 19.  What bounds it: per pass a grid barrier of 2.7 k cycles, 1.5 k of
+// N = 19 (the passes launched one by one; chained, N=20 forward, p=5, takes
+// 12 us less).  What bounds it: per pass a grid barrier of 2.7 k cycles, 1.5 k of
 // loads and stores, and the rounds (as in fq_small.cuh).
 #pragma once
 

@@ -134,7 +134,20 @@ struct PassArgs {
     int* err;        // device error flag (bounded waits that gave up)
     int mir;         // mirror pass of a half state (k_pass, k_pass_dual with MIR)
     int full;        // write both halves of the state (ST = 2)
+    int chained;     // 1: first pass of a chain, 2: follows the pass before it (chain_pass)
 };
+
+// Passes of a chain (see chain_pass in fq_engine.cu).  A pass may start once
+// every CTA of the pass before it has come this far, so its CTAs take the SMs
+// as those leave them, with the launch, the copy of the cut tables and the
+// address set-up behind them.  Nothing but tables and weights is touched
+// before the wait: they were complete when the chain's first pass, an
+// ordinary launch, began.  The wait ends when the pass before it is complete
+// and its writes can be read, and so, in turn, all passes before that one.
+__device__ __forceinline__ void pass_chain() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ int tile_phys(int j, int l, int a) { return j < l ? j : a + j - l; }
 
@@ -821,6 +834,7 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
             ct.template setup<PH != PH_NONE>(sw, N, l, a, tid, A.gamma);
         __syncthreads();  // the weights in the buffer are dead from here on
     }
+    if (A.chained) pass_chain();
 
     // Address pieces: the thread's offsets in layouts L0 and L1 and the
     // strides of the 4 register bits of each (uniform across the grid).

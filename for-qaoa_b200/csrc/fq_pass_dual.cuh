@@ -186,6 +186,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         ct.template setup<true>(sw, N, l, a, tid, A.gamma);
         __syncthreads();  // the weights in buf are dead from here on
     }
+    if (A.chained) pass_chain();
 
     const i64 thr_off = tile_off(tid, l, a);
     const i64 thr_off1 = tile_off(lay_index<1>(tid, 0), l, a);

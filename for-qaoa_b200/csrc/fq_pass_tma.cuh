@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
         for (int i = tid; i < N * N; i += kPassThreads) sw[i] = gw[i];
     }
     if (PH != PH_NONE && INTW) load_phase_tables(A, smtab, tid, kPassThreads);
+    if (A.chained) pass_chain();
     __syncthreads();
     if (tid == 0)
         for (i64 j = 0; j < kStages - 1 && j < my_tiles; j++) issue(j);

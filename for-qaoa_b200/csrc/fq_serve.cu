@@ -541,6 +541,11 @@ int fq_server_create(int device, double hbm_budget_bytes, int lanes, fq_server**
         if (cudaStreamCreateWithPriority(&L.st, cudaStreamNonBlocking, prio_low) != cudaSuccess)
             st = FQ_ERR_CUDA;
         if (st == FQ_OK) st = fq_ctx_create(device, L.st, &L.ctx);
+        // CTAs of a chained pass that wait for the pass before it hold SMs
+        // that the other lanes could use: a burst of 96 requests of 10 to 20
+        // qubits took 3.58 ms with chains, 3.48 without (whole burst, A/B in
+        // one call).
+        if (st == FQ_OK) L.ctx->chain = false;
         if (st == FQ_OK &&
             cudaEventCreateWithFlags(&L.done, cudaEventDisableTiming) != cudaSuccess)
             st = FQ_ERR_CUDA;
