@@ -49,6 +49,18 @@ double now_s() {
 
 size_t session_bytes(int N) { return 2 * (sizeof(double2) << N); }
 
+// The work before an event: any status but done and not-ready means that it
+// failed, and its results are not to be read.
+enum class Work { running, done, failed };
+Work work_of(cudaEvent_t e) {
+    const cudaError_t q = cudaEventQuery(e);
+    if (q == cudaSuccess) return Work::done;
+    if (q == cudaErrorNotReady) return Work::running;
+    cudaGetLastError();
+    set_error("device work failed: %s", cudaGetErrorString(q));
+    return Work::failed;
+}
+
 struct Req {
     uint64_t ticket = 0, session = 0;
     int N = 0, P = 0;
@@ -253,13 +265,17 @@ struct fq_server {
     }
 
     // All of a batch's results under one lock: the clients submit meanwhile.
-    void complete_batch(Batch& B) {
+    void complete_batch(Batch& B, int st) {
+        if (st != FQ_OK) {
+            fail(st);
+            cudaStreamSynchronize(B.st);  // its buffers are free for the next batch
+        }
         std::vector<fq_result> res;
         res.reserve(B.reqs.size());
         for (size_t i = 0; i < B.reqs.size(); i++) {
             const Req& r = B.reqs[i];
             const double* out = B.out + B.out_off[i];
-            res.push_back(result_of(r, FQ_OK, out, out + 1, out + 1 + r.P, B.t_start));
+            res.push_back(result_of(r, st, out, out + 1, out + 1 + r.P, B.t_start));
         }
         B.reqs.clear();
         B.busy = false;
@@ -416,9 +432,12 @@ struct fq_server {
         }
     }
 
-    void complete_large(Lane& L) {
+    void complete_large(Lane& L, int st) {
         double e = 0, gg[FQ_SERVE_MAX_LAYERS], gb[FQ_SERVE_MAX_LAYERS];
-        const int st = grad_collect(L.ctx, L.cur.N, L.cur.P, &e, gg, gb);
+        if (st == FQ_OK)
+            st = grad_collect(L.ctx, L.cur.N, L.cur.P, &e, gg, gb);
+        else
+            cudaStreamSynchronize(L.st);  // before the session's buffers change hands
         if (st != FQ_OK) fail(st);
         end_step(L.cur.session);
         finish(L.cur, st, &e, gg, gb, L.cur.t_start);
@@ -452,13 +471,8 @@ struct fq_server {
                 continue;
             }
             const double t0 = now_s();
-            while (true) {
-                const cudaError_t q = cudaEventQuery(L.done);
-                if (q == cudaSuccess) break;
-                if (q != cudaErrorNotReady) {
-                    cudaGetLastError();
-                    break;  // grad_collect reports the failure
-                }
+            Work w;
+            while ((w = work_of(L.done)) == Work::running) {
                 // A 20 us sleep takes 70 or more, as long as a request of up to
                 // 20 qubits: those are polled (yielding) for their first half
                 // millisecond.
@@ -467,7 +481,7 @@ struct fq_server {
                 else
                     std::this_thread::sleep_for(std::chrono::microseconds(20));
             }
-            complete_large(L);
+            complete_large(L, w == Work::done ? FQ_OK : FQ_ERR_CUDA);
             cv_lane.notify_all();  // the session may have a next step queued
         }
     }
@@ -479,8 +493,9 @@ struct fq_server {
         while (true) {
             bool worked = false, pending = false;
             for (auto& B : batches) {
-                if (B.busy && cudaEventQuery(B.done) == cudaSuccess) {
-                    complete_batch(B);
+                const Work w = B.busy ? work_of(B.done) : Work::running;
+                if (w != Work::running) {
+                    complete_batch(B, w == Work::done ? FQ_OK : FQ_ERR_CUDA);
                     worked = true;
                 }
                 if (!B.busy) {
