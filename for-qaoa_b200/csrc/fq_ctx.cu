@@ -27,11 +27,20 @@ int validate_ctx(fq_ctx* ctx) {
     return FQ_OK;
 }
 
+static int reset_counter(fq_ctx* ctx) {
+    FQ_CUDA(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
+    FQ_CUDA(cudaStreamSynchronize(ctx->stream));
+    return FQ_OK;
+}
+
 int check_device_error(fq_ctx* ctx) {
     const int flag = *(volatile int*)ctx->err;
     if (flag) {
         *(volatile int*)ctx->err = 0;
-        ctx->counter_lost = true;
+        // A grid barrier that gave up has not counted all its arrivals.  The
+        // stream is idle here, and later launches, replays of captured ones
+        // among them, have no reset of their own.
+        FQ_TRY(reset_counter(ctx));
         set_error("a device-side bounded wait gave up (flag %d); results are incomplete", flag);
         return FQ_ERR_TIMEOUT;
     }
@@ -217,7 +226,6 @@ int fq_ctx_create(int device, void* stream, fq_ctx** out) {
             break;
         }
         c->tcut_bytes = kTcutBytes;
-        c->counter_lost = true;  // zeroed by the first launch that uses it
         c->h_stage_bytes = std::max(wbytes, (size_t)256 * 1024);
         if (cudaMallocHost(&c->h_stage, c->h_stage_bytes) != cudaSuccess ||
             cudaMallocHost(&c->result, sizeof(double) * kResultWords + 64) != cudaSuccess) {
@@ -231,6 +239,8 @@ int fq_ctx_create(int device, void* stream, fq_ctx** out) {
             break;
         }
         if (cudaEventRecord(c->stage_evt, c->stream) != cudaSuccess) { st = FQ_ERR_CUDA; break; }
+        // Zeroed now: the first launch that counts on it may be a captured one.
+        if (reset_counter(c) != FQ_OK) { st = FQ_ERR_CUDA; break; }
     } while (0);
     if (st != FQ_OK) {
         set_error("context creation failed: %s", cudaGetErrorString(cudaGetLastError()));

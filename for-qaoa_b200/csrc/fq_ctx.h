@@ -28,7 +28,6 @@ struct fq_ctx {
     long long tcut_version = -1;  // g_version the tables were built for (-1: none)
     int tcut_n = -1;              // and N
     unsigned* d_counter = nullptr;   // grid barrier of k_mid: arrivals so far
-    bool counter_lost = false;       // not known to be between two launches' (see run_mid)
     bool cooperative = false;        // the device takes cooperative launches
     unsigned char* d_img = nullptr;  // static cut tables of the plan's geometries, built with them
     int partial_cap = 0;

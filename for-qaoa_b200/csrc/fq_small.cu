@@ -138,10 +138,6 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
     a.partial = ctx->d_partial;
     a.counter = ctx->d_counter;
     a.err = ctx->err;
-    if (ctx->counter_lost) {  // a barrier gave up: its arrivals are not all counted
-        FQ_CUDA(cudaMemsetAsync(ctx->d_counter, 0, sizeof(unsigned), ctx->stream));
-        ctx->counter_lost = false;
-    }
     const void* fn = grad ? (const void*)k_mid<true> : (const void*)k_mid<false>;
     // Only the tables the job has: instances of other lanes fit beside it.
     const size_t smem = mid_smem_bytes(nb, grad, a.job.ntab * (a.job.keep ? P : 1));

@@ -31,11 +31,12 @@ static void note(const char* fmt, ...) {
     va_end(ap);
 }
 static int forbidden(void) { return capture && capture_mode != 2 ? CAPTURE_UNSUPPORTED : OK; }
-static int launch(const char* how, const void* fn) {
+static int launch(const void* fn, void** args) {
     const char* name = "?";
     for (int i = 0; i < nkernels; i++)
         if (kernels[i].fn == fn) name = kernels[i].name;
-    note("%s %s%s\n", how, name, capture ? " captured" : "");
+    if (strstr(name, "k_selftest_wait")) **(int**)args[0] = 2; /* all that it does */
+    note("launch %s%s\n", name, capture ? " captured" : "");
     return OK;
 }
 
@@ -72,16 +73,16 @@ int __cudaPopCallConfiguration(dim* g, dim* b, size_t* smem, void** s) {
     return OK;
 }
 int cudaLaunchKernel(const void* fn, dim g, dim b, void** a, size_t m, void* s) {
-    (void)g, (void)b, (void)a, (void)m, (void)s;
-    return launch("launch", fn);
+    (void)g, (void)b, (void)m, (void)s;
+    return launch(fn, a);
 }
 int cudaLaunchCooperativeKernel(const void* fn, dim g, dim b, void** a, size_t m, void* s) {
-    (void)g, (void)b, (void)a, (void)m, (void)s;
-    return launch("launch", fn);
+    (void)g, (void)b, (void)m, (void)s;
+    return launch(fn, a);
 }
 int cudaLaunchKernelExC(const void* cfg, const void* fn, void** a) {
-    (void)cfg, (void)a;
-    return launch("launch", fn);
+    (void)cfg;
+    return launch(fn, a);
 }
 int cudaFuncSetAttribute(const void* fn, int a, int v) { (void)fn, (void)a, (void)v; return OK; }
 

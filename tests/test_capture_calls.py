@@ -1,0 +1,34 @@
+"""CPU tests, over a CUDA runtime without a device, of what calls under
+stream capture leave to the graph and what is done at once."""
+import fake_cuda
+
+BARRIER = """
+ctx = fq.Context(0)
+made = log()
+st = ctx.state(17)
+def circuit():
+    log()
+    ctx.qaoa_forward(st, graph(17), [0.1, 0.2], [0.3, 0.4], energy=False)
+    return log()
+# The grid barrier's counter is zeroed with the context, and waited for.
+zero = [i for i, x in enumerate(made) if x == "memset"]
+assert zero and "sync" in made[zero[-1]:], made
+# Captured first, then called: neither run depends on the other's reset.
+fake.fake_capture(1)
+captured = circuit()
+fake.fake_capture(0)
+assert [x.split()[0] for x in captured] == ["launch"], captured
+assert [x.split()[0] for x in circuit()] == ["launch"]
+# A wait that gave up: the counter is reset when the host hears of it, not by
+# the next launch, which may be the replay of a captured one.
+log()
+assert fq.lib().fq_ctx_selftest_wait(ctx.handle) == fq.OK
+assert fq.lib().fq_ctx_synchronize(ctx.handle) == fq.ERR_TIMEOUT
+reset = log()
+assert "memset" in reset and reset[-1] == "sync", reset
+print("ok")
+"""
+
+
+def test_barrier_counter_is_ready_at_every_launch(tmp_path):
+    assert "ok" in fake_cuda.run(BARRIER, tmp_path)

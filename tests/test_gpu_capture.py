@@ -1,0 +1,49 @@
+"""Circuits captured in a CUDA graph as the first call of their context,
+called as usual before the graph runs, and replayed in turn with calls:
+always the oracle's state."""
+import numpy as np
+import pytest
+
+from conftest import angles, assert_state_close, complete_int
+
+pytestmark = pytest.mark.gpu
+
+
+class Captured:
+    def __init__(self, ctx, stream, st, W, g, b):
+        import torch
+        self.graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(self.graph, stream=stream):
+            ctx.qaoa_forward(st, W, g, b, energy=False)
+
+    def replay(self):
+        import torch
+        self.graph.replay()
+        torch.cuda.synchronize()
+
+
+def context(fq):
+    import torch
+    stream = torch.cuda.Stream()
+    return stream, fq.Context(0, stream.cuda_stream)
+
+
+@pytest.mark.parametrize("n", [16, 17, 19])
+def test_capture_is_the_first_call(fq, oracle, n):
+    rng = np.random.default_rng(n)
+    W, (g, b) = complete_int(n, rng), angles(rng, 3)
+    want = oracle.qaoa_logical(W, g, b)
+    stream, ctx = context(fq)
+    with ctx as c:
+        st = c.state(n)
+        try:
+            cap = Captured(c, stream, st, W, g, b)
+            for _ in range(2):
+                c.qaoa_forward(st, W, g, b)
+                assert_state_close(st.to_host(), want, what=f"N={n}, called")
+                st.init_basis0()
+                c.synchronize()
+                cap.replay()
+                assert_state_close(st.to_host(), want, what=f"N={n}, replayed")
+        finally:
+            st.free()
