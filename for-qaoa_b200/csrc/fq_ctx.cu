@@ -9,6 +9,7 @@
 
 #include "fq_ctx.h"
 #include "fq_pass.cuh"
+#include "fq_small.h"
 
 namespace fq {
 
@@ -24,6 +25,27 @@ void set_error(const char* fmt, ...) {
 int validate_ctx(fq_ctx* ctx) {
     FQ_CHECK(ctx != nullptr, FQ_ERR_INVALID, "null context");
     FQ_CUDA(cudaSetDevice(ctx->device));
+    return FQ_OK;
+}
+
+constexpr int kPutWords = 500;  // 4000 bytes of parameters
+struct PutWords {
+    double w[kPutWords];
+};
+
+__global__ void k_put(const __grid_constant__ PutWords p, double* dst, int n) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = p.w[i];
+}
+
+int put_words(fq_ctx* ctx, double* dst, const double* host, size_t n) {
+    for (size_t i = 0; i < n; i += kPutWords) {
+        PutWords p;
+        const int k = (int)std::min<size_t>(n - i, kPutWords);
+        memcpy(p.w, host + i, k * sizeof(double));
+        k_put<<<1, 128, 0, ctx->stream>>>(p, dst + i, k);
+        FQ_CUDA(cudaGetLastError());
+        ctx->launches++;
+    }
     return FQ_OK;
 }
 
@@ -221,11 +243,13 @@ int fq_ctx_create(int device, void* stream, fq_ctx** out) {
             cudaMalloc(&c->d_partial, sizeof(double) * c->partial_cap) != cudaSuccess ||
             cudaMalloc(&c->d_tcut, kTcutBytes) != cudaSuccess ||
             cudaMalloc(&c->d_img, kMaxGeoms * kImgStride) != cudaSuccess ||
+            cudaMalloc(&c->d_job, sizeof(double) * kJobWords) != cudaSuccess ||
             cudaMalloc(&c->d_counter, sizeof(unsigned)) != cudaSuccess) {
             st = FQ_ERR_OOM;
             break;
         }
         c->tcut_bytes = kTcutBytes;
+        c->job_words = kJobWords;
         c->h_stage_bytes = std::max(wbytes, (size_t)256 * 1024);
         if (cudaMallocHost(&c->h_stage, c->h_stage_bytes) != cudaSuccess ||
             cudaMallocHost(&c->result, sizeof(double) * kResultWords + 64) != cudaSuccess) {
@@ -261,6 +285,8 @@ int fq_ctx_destroy(fq_ctx* c) {
     cudaFree(c->d_tcut);
     cudaFree(c->d_img);
     cudaFree(c->d_counter);
+    cudaFree(c->d_job);
+    for (void* p : c->retired) cudaFree(p);
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->result) cudaFreeHost(c->result);
     if (c->stage_evt) cudaEventDestroy(c->stage_evt);

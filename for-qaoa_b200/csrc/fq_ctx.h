@@ -31,6 +31,9 @@ struct fq_ctx {
     bool cooperative = false;        // the device takes cooperative launches
     unsigned char* d_img = nullptr;  // static cut tables of the plan's geometries, built with them
     int partial_cap = 0;
+    double* d_job = nullptr;  // data of one deep small instance (run_small), job_words of room
+    size_t job_words = 0;
+    std::vector<void*> retired;  // outgrown buffers: launches in flight or captured still read them
     // Pinned host staging (uploads of weights and small tables).
     unsigned char* h_stage = nullptr;
     size_t h_stage_bytes = 0;
@@ -77,6 +80,9 @@ struct GraphPrep {
 int prep_graph(const double* upper, int N, GraphPrep& g);
 // Uploads the graph's weights to ctx->d_w (skipped when unchanged).
 int upload_graph(fq_ctx* ctx, const GraphPrep& g, const double* upper);
+// Enqueues n words for device memory at dst.  They travel in kernel parameters,
+// so host may change at once and a captured call keeps the words it was given.
+int put_words(fq_ctx* ctx, double* dst, const double* host, size_t n);
 // Waits until the pinned staging buffer can be rewritten.
 int stage_acquire(fq_ctx* ctx);
 int validate_ctx(fq_ctx* ctx);

@@ -153,6 +153,23 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
     return FQ_OK;
 }
 
+// Room for `words` in ctx->d_job (forward circuits of more than 2048 layers
+// outgrow it), also during a capture.
+static int job_buffer(fq_ctx* ctx, size_t words) {
+    if (words <= ctx->job_words) return FQ_OK;
+    words = std::max(words, 2 * ctx->job_words);  // so the outgrown ones stay below the last
+    double* d = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    FQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaMalloc(&d, words * sizeof(double));
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    FQ_CUDA(e);
+    ctx->retired.push_back(ctx->d_job);
+    ctx->d_job = d;
+    ctx->job_words = words;
+    return FQ_OK;
+}
+
 int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
               int flags, double2* state, double* out) {
     const int c = small_class(g.N), words = small_words(g.N, P);
@@ -167,30 +184,22 @@ int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, cons
         FQ_TRY(grad ? launch_any<true>(c, &a, nullptr, 1, ctx->stream)
                     : launch_any<false>(c, &a, nullptr, 1, ctx->stream));
     } else {
-        // Deep circuits: descriptor and data through device memory.
-        std::vector<double> h((sizeof(SmallJob) + 7) / 8 + words);
-        double* const data = h.data() + (h.size() - words);
+        // Deep circuits: descriptor and data through the context's buffer.
+        std::vector<double> h(job_words(g.N, P));
+        FQ_TRY(job_buffer(ctx, h.size()));
+        const size_t at = h.size() - words;
         SmallJob J;
         small_job(g, P, gammas, betas, flags, small_table_cap(c, false), small_table_most(g.N), J,
-                  data);
-        void* d = nullptr;
-        FQ_CUDA(cudaMalloc(&d, h.size() * sizeof(double)));
-        J.w = (const double*)d + (h.size() - words);
+                  h.data() + at);
+        J.w = ctx->d_job + at;
         J.lay = J.w + g.N * (g.N - 1) / 2;
         J.out = out;
         J.state = state;
         memcpy(h.data(), &J, sizeof(J));
-        int st = FQ_OK;
-        if (cudaMemcpyAsync(d, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice,
-                            ctx->stream) != cudaSuccess)
-            st = FQ_ERR_CUDA;
-        if (st == FQ_OK)
-            st = grad ? launch_any<true>(c, nullptr, (const SmallJob*)d, 1, ctx->stream)
-                      : launch_any<false>(c, nullptr, (const SmallJob*)d, 1, ctx->stream);
-        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
-        cudaFree(d);
-        FQ_TRY(st);
-        FQ_CUDA(e);
+        FQ_TRY(put_words(ctx, ctx->d_job, h.data(), h.size()));
+        const SmallJob* const d = (const SmallJob*)ctx->d_job;
+        FQ_TRY(grad ? launch_any<true>(c, nullptr, d, 1, ctx->stream)
+                    : launch_any<false>(c, nullptr, d, 1, ctx->stream));
     }
     prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
     ctx->launches++;

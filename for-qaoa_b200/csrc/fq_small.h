@@ -31,6 +31,14 @@ struct SmallJob {
 // Data words of a job behind its descriptor.
 __host__ __device__ inline int small_words(int N, int P) { return N * (N - 1) / 2 + 4 * P; }
 
+// Words of a job in device memory: descriptor, then data.
+__host__ __device__ inline size_t job_words(int N, int P) {
+    return (sizeof(SmallJob) + 7) / 8 + (size_t)small_words(N, P);
+}
+// Room every context has: any gradient's (1 + 2P results of kResultWords).
+constexpr size_t kJobWords = (sizeof(SmallJob) + 7) / 8 +
+                             kSmallJobMaxQubits * (kSmallJobMaxQubits - 1) / 2 + 4 * 2048;
+
 // Size class of an N-qubit instance: 0..3 for one CTA of 2^(8..11)
 // amplitudes (a half state from N = 9 on), 4..6 for clusters of 2, 4, 8.
 constexpr int kSmallClasses = 7;

@@ -32,3 +32,32 @@ print("ok")
 
 def test_barrier_counter_is_ready_at_every_launch(tmp_path):
     assert "ok" in fake_cuda.run(BARRIER, tmp_path)
+
+
+DEEP = """
+ctx = fq.Context(0)
+states = {n: ctx.state(n) for n in (2, 9, 12, 15)}
+def circuit(n, P):
+    log()
+    ctx.qaoa_forward(states[n], graph(n), [0.1] * P, [0.3] * P, energy=False)
+    return log()
+for n, P in ((9, 60), (12, 64), (15, 40), (2, 1000), (15, 2047)):
+    called = circuit(n, P)
+    fake.fake_capture(1)
+    captured = circuit(n, P)
+    fake.fake_capture(0)
+    assert all(x.startswith("launch ") for x in called), (n, P, called)
+    assert [x + " captured" for x in called] == captured, (n, P, captured)
+fake.fake_capture(1)
+grown = circuit(9, 5000)
+fake.fake_capture(0)
+assert grown[0] == "malloc" and all(x.endswith(" captured") for x in grown[1:]), grown
+ctx.close()
+print("ok")
+"""
+
+
+def test_deep_small_circuits_neither_wait_nor_allocate(tmp_path):
+    """More layers than the kernel parameters hold: only launches, captured or
+    not (but for growth beyond what every context has room for)."""
+    assert "ok" in fake_cuda.run(DEEP, tmp_path)

@@ -47,3 +47,24 @@ def test_capture_is_the_first_call(fq, oracle, n):
                 assert_state_close(st.to_host(), want, what=f"N={n}, replayed")
         finally:
             st.free()
+
+
+@pytest.mark.parametrize("n,P", [(9, 60), (12, 44), (14, 36), (15, 33), (3, 2100)])
+def test_deep_small_circuits(fq, oracle, n, P):
+    """More layers than the kernel parameters hold (and, last, than every
+    context has room for): captured, replayed between calls of other circuits."""
+    rng = np.random.default_rng(n)
+    (W, V), (g, b) = (complete_int(n, rng) for _ in range(2)), angles(rng, P)
+    want, other = oracle.qaoa_logical(W, g, b), oracle.qaoa_logical(V, b, g)
+    stream, ctx = context(fq)
+    with ctx as c:
+        st = c.state(n)
+        try:
+            cap = Captured(c, stream, st, W, g, b)
+            for _ in range(2):
+                c.qaoa_forward(st, V, b, g)
+                assert_state_close(st.to_host(), other, what=f"N={n}, called")
+                cap.replay()
+                assert_state_close(st.to_host(), want, what=f"N={n}, replayed")
+        finally:
+            st.free()
