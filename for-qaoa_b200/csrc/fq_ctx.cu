@@ -119,8 +119,29 @@ int prep_graph(const double* upper, int N, GraphPrep& g) {
     return FQ_OK;
 }
 
+cudaError_t alloc_any_time(void** p, size_t bytes) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return e;
+}
+
 int upload_graph(fq_ctx* ctx, const GraphPrep& g, const double* upper) {
     const size_t nn = (size_t)g.N * g.N;
+    cudaStreamCaptureStatus cap;
+    FQ_CUDA(cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) ctx->captured = true;
+    if (ctx->captured) {
+        std::vector<double> w(g.integer ? (nn + 1) / 2 : nn);
+        memcpy(w.data(), g.integer ? (const void*)g.wi.data() : (const void*)g.wd.data(),
+               nn * (g.integer ? sizeof(int) : sizeof(double)));
+        FQ_TRY(put_words(ctx, (double*)ctx->d_w, w.data(), w.size()));
+        ctx->g_version++;
+        return FQ_OK;
+    }
     // Key: the upper triangle plus the path taken.
     if (ctx->g_n == g.N && ctx->g_key.size() == nn + 1 &&
         memcmp(ctx->g_key.data(), upper, nn * sizeof(double)) == 0 &&

@@ -38,6 +38,10 @@ struct fq_ctx {
     unsigned char* h_stage = nullptr;
     size_t h_stage_bytes = 0;
     cudaEvent_t stage_evt = nullptr;
+    // Calls of this context were captured.  Their graphs carry the weights and
+    // rebuild the tables, so a replay leaves its own in the buffers: what the
+    // last call left there is not relied on any more.
+    bool captured = false;
     // Graph cache: the last weights uploaded to d_w.
     std::vector<double> g_key;
     int g_n = -1;
@@ -78,11 +82,14 @@ struct GraphPrep {
 };
 
 int prep_graph(const double* upper, int N, GraphPrep& g);
-// Uploads the graph's weights to ctx->d_w (skipped when unchanged).
+// Uploads the graph's weights to ctx->d_w (skipped when unchanged, unless calls
+// of this context are or were captured).
 int upload_graph(fq_ctx* ctx, const GraphPrep& g, const double* upper);
 // Enqueues n words for device memory at dst.  They travel in kernel parameters,
 // so host may change at once and a captured call keeps the words it was given.
 int put_words(fq_ctx* ctx, double* dst, const double* host, size_t n);
+// cudaMalloc, also during a capture; a failure is not left behind as the last error.
+cudaError_t alloc_any_time(void** p, size_t bytes);
 // Waits until the pinned staging buffer can be rewritten.
 int stage_acquire(fq_ctx* ctx);
 int validate_ctx(fq_ctx* ctx);

@@ -449,18 +449,18 @@ static int tile_cut_tables(fq_ctx* ctx, const GraphPrep& g, int N,
     }
     ctx->tcut_version = -1;
     if (need > ctx->tcut_bytes) {
-        if (ctx->d_tcut) {
+        if (ctx->d_tcut && ctx->captured) {
+            ctx->retired.push_back(ctx->d_tcut);  // captured calls still use it
+        } else if (ctx->d_tcut) {
             FQ_CUDA(cudaStreamSynchronize(ctx->stream));
             FQ_CUDA(cudaFree(ctx->d_tcut));
-            ctx->d_tcut = nullptr;
-            ctx->tcut_bytes = 0;
         }
-        if (cudaMalloc(&ctx->d_tcut, need) != cudaSuccess) {
-            cudaGetLastError();  // clear the allocation failure
-            ctx->d_tcut = nullptr;
-        } else {
+        ctx->d_tcut = nullptr;
+        ctx->tcut_bytes = 0;
+        if (alloc_any_time(&ctx->d_tcut, need) == cudaSuccess)
             ctx->tcut_bytes = need;
-        }
+        else
+            ctx->d_tcut = nullptr;
     }
     const bool fits = need <= ctx->tcut_bytes;
     const i64 nt = fits ? ntiles : 0;

@@ -158,14 +158,10 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
 static int job_buffer(fq_ctx* ctx, size_t words) {
     if (words <= ctx->job_words) return FQ_OK;
     words = std::max(words, 2 * ctx->job_words);  // so the outgrown ones stay below the last
-    double* d = nullptr;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    FQ_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    const cudaError_t e = cudaMalloc(&d, words * sizeof(double));
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    FQ_CUDA(e);
+    void* d = nullptr;
+    FQ_CUDA(alloc_any_time(&d, words * sizeof(double)));
     ctx->retired.push_back(ctx->d_job);
-    ctx->d_job = d;
+    ctx->d_job = (double*)d;
     ctx->job_words = words;
     return FQ_OK;
 }

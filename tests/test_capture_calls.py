@@ -61,3 +61,37 @@ def test_deep_small_circuits_neither_wait_nor_allocate(tmp_path):
     """More layers than the kernel parameters hold: only launches, captured or
     not (but for growth beyond what every context has room for)."""
     assert "ok" in fake_cuda.run(DEEP, tmp_path)
+
+
+TABLES = """
+ctx = fq.Context(0)
+st = {n: ctx.state(n) for n in (20, 21, 26)}
+def circuit(n, captured=False, seed=1):
+    fake.fake_capture(int(captured))
+    log()
+    ctx.qaoa_forward(st[n], graph(n, seed), [0.1, 0.2], [0.3, 0.4], energy=False)
+    fake.fake_capture(0)
+    out = log()
+    assert all(("captured" in x) == captured for x in out if x != "malloc"), out
+    return {"weights": any("k_put" in x or x.startswith("copy") for x in out),
+            "tables": any("k_tile_cuts" in x for x in out), "free": "free" in out}
+kept = dict(weights=False, tables=False, free=False)
+made = dict(weights=True, tables=True, free=False)
+assert circuit(20) == made and circuit(20) == kept
+assert circuit(20, seed=2) == made
+# The weights are in place (as any other call on the graph leaves them), the
+# tables are another size's; then the first circuit is captured.
+ctx.cost_phase(st[21], 0.1, graph(21), True, 0.5)
+assert circuit(21, captured=True) == made
+for _ in range(2):
+    assert circuit(21) == made  # whether or not the graph has run
+assert circuit(21, captured=True) == made
+assert circuit(26) == made  # the tables grow, the captured calls keep theirs
+assert circuit(26, captured=True) == made
+ctx.close()
+print("ok")
+"""
+
+
+def test_captured_circuits_carry_weights_and_tables(tmp_path):
+    assert "ok" in fake_cuda.run(TABLES, tmp_path)

@@ -68,3 +68,33 @@ def test_deep_small_circuits(fq, oracle, n, P):
                 assert_state_close(st.to_host(), want, what=f"N={n}, replayed")
         finally:
             st.free()
+
+
+@pytest.mark.parametrize("n,P", [(16, 65), (20, 3), (21, 2)])
+def test_replays_between_calls_on_other_graphs(fq, oracle, n, P):
+    """Circuits as passes with tables (16 qubits: more layers than one launch
+    holds): captured with only the weights in place, replayed between calls
+    on another graph, and after the tables' buffer has been outgrown."""
+    rng = np.random.default_rng(n + P)
+    (W, V), (g, b) = (complete_int(n, rng) for _ in range(2)), angles(rng, P)
+    want, other = oracle.qaoa_logical(W, g, b), oracle.qaoa_logical(V, g, b)
+    big, (G, B) = complete_int(25, rng), angles(rng, 1)
+    stream, ctx = context(fq)
+    with ctx as c:
+        st, st25 = c.state(n), c.state(25)
+        try:
+            st.init_basis0()
+            c.expectation(st, W)  # the weights, nothing else
+            cap = Captured(c, stream, st, W, g, b)
+            c.qaoa_forward(st, W, g, b)
+            assert_state_close(st.to_host(), want, what=f"N={n}, called first")
+            for k in range(3):
+                c.qaoa_forward(st, V, g, b)
+                assert_state_close(st.to_host(), other, what=f"N={n}, called")
+                if k == 1:
+                    c.qaoa_forward(st25, big, G, B)
+                cap.replay()
+                assert_state_close(st.to_host(), want, what=f"N={n}, replayed")
+        finally:
+            st.free()
+            st25.free()
