@@ -33,14 +33,10 @@ __global__ void k_phase_table(double2* tab, int cmin, int n, long long W, double
 // passes: tab[j] = z^j for j < 32, tab[32 + h] = z^(dlo + 32h).
 __global__ void k_phase_table2(double2* tab, int dlo, int nhi, double gamma) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    double sn, cs;
-    if (i < kPhaseLo) {
-        sincos(gamma * (double)i, &sn, &cs);
-        tab[i] = make_double2(cs, sn);
-    } else if (i < kPhaseLo + nhi) {
-        sincos(gamma * (double)(dlo + 32ll * (i - kPhaseLo)), &sn, &cs);
-        tab[i] = make_double2(cs, sn);
-    }
+    if (i < kPhaseLo)
+        tab[i] = unit_power(gamma, (double)i);
+    else if (i < kPhaseLo + nhi)
+        tab[i] = unit_power(gamma, (double)(dlo + 32ll * (i - kPhaseLo)));
 }
 
 // Tables of k_phase_table2 for up to kMaxTableLayers layers in one launch:
@@ -57,20 +53,16 @@ __global__ void k_phase_tables2(double2* tab, int dlo, int nhi, LayerGammas lg, 
     const int p = blockIdx.y;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
-    double sn, cs;
     double2* t = tab + (size_t)p * kTableStride;
     if (blockIdx.x == gridDim.x - 1) {
         const int j = threadIdx.x;
         if (j >= ngeom * kQtabStride) return;
         const WT* creg = reinterpret_cast<const WT*>(img + (j / kQtabStride) * kImgStride);
-        sincos(lg.g[p] * (double)creg[j % kQtabStride], &sn, &cs);
-        t[kPhaseLo + kPhaseHiMax + j] = make_double2(cs, sn);
+        t[kPhaseLo + kPhaseHiMax + j] = unit_power(lg.g[p], (double)creg[j % kQtabStride]);
     } else if (i < kPhaseLo) {
-        sincos(lg.g[p] * (double)i, &sn, &cs);
-        t[i] = make_double2(cs, sn);
+        t[i] = unit_power(lg.g[p], (double)i);
     } else if (i < kPhaseLo + nhi) {
-        sincos(lg.g[p] * (double)(dlo + 32ll * (i - kPhaseLo)), &sn, &cs);
-        t[i] = make_double2(cs, sn);
+        t[i] = unit_power(lg.g[p], (double)(dlo + 32ll * (i - kPhaseLo)));
     }
 }
 
@@ -366,9 +358,11 @@ void set_table_args(PassArgs& A, const GraphPrep& g, double gamma, double scale)
         table_range(g, dlo, dhi);
         A.dlo = (int)dlo;
         A.ntab = (int)(dhi - dlo + 1);
-        const double th = -gamma * (double)g.W_int / 2;
-        A.ph0x = scale * cos(th);
-        A.ph0y = scale * sin(th);
+        // exp(-i*gamma*W/2), turned by the product's rounding error (unit_power).
+        const double W = (double)g.W_int, x = gamma * W, lo = fma(gamma, W, -x) / 2;
+        const double c = cos(x / 2), s = sin(x / 2);
+        A.ph0x = scale * (c - s * lo);
+        A.ph0y = -scale * (s + c * lo);
     }
 }
 

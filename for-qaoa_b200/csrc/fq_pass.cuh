@@ -162,6 +162,19 @@ constexpr int kTableStride = kPhaseLo + kPhaseHiMax + kMaxGeoms * kQtabStride;
 constexpr int kMaxTableLayers = 64;
 static_assert(kTableStride * kMaxTableLayers <= kMaxPhaseTable, "layer tables fit the buffer");
 
+// exp(i*g*v), the product's rounding error (exact, by fma) added to its angle.
+// A cut of a thousand times an angle of pi is rounded by 2e-13, the same in
+// every amplitude that takes the table's entry, so sums over the state do not
+// average it out.  Integer weights, N = 20..22, against 80-bit arithmetic
+// (median of 20 to 40 instances): states 1.1e-13 -> 2e-15, gradients 0.8e-13
+// to 1.2e-13 -> 1e-14 of their largest entry.
+__device__ __forceinline__ double2 unit_power(double g, double v) {
+    const double x = __dmul_rn(g, v), lo = fma(g, v, -x);
+    double sn, cs;
+    sincos(x, &sn, &cs);
+    return make_double2(fma(-lo, sn, cs), fma(lo, cs, sn));
+}
+
 // Shared-memory bytes reserved for the two-level phase table.
 __host__ __device__ inline size_t phase_smem_bytes() {
     return sizeof(double2) * (kPhaseLo + kPhaseHiMax);
@@ -615,9 +628,7 @@ struct CutTables {
     }
 
     __device__ void qtab_entry(int i, double gamma) const {
-        double sn, cs;
-        sincos(gamma * (double)creg[i], &sn, &cs);
-        qtab[i] = make_double2(cs, sn);
+        qtab[i] = unit_power(gamma, (double)creg[i]);
     }
 
     // Tile bit of register bit k and of thread bit j in layout L (L0: the

@@ -204,17 +204,13 @@ __global__ void __launch_bounds__(kColThreads, 1)
             reinterpret_cast<const WT*>(img + (PS::thrc - PS::creg)) + 5 * kPassThreads;
         const int t = threadIdx.x & (kPassThreads - 1), ln = t & 31;
         const int t1 = (t >> 5) | ((ln & 1) << 3) | ((ln >> 1) << 4);
-        for (int k = threadIdx.x >> 8; k < 4; k += 2) {
-            double sn, cs;
-            sincos(A.gamma * (double)ithr[(1 + k) * kPassThreads + t1], &sn, &cs);
-            zf[k * kPassThreads + t] = make_double2(cs, sn);
-        }
+        for (int k = threadIdx.x >> 8; k < 4; k += 2)
+            zf[k * kPassThreads + t] =
+                unit_power(A.gamma, (double)ithr[(1 + k) * kPassThreads + t1]);
         if (threadIdx.x < kPassThreads) cthr[t] = ithr[t1];
         if (threadIdx.x < 16) {
             creg[threadIdx.x] = icreg[threadIdx.x];
-            double sn, cs;
-            sincos(A.gamma * (double)icreg[threadIdx.x], &sn, &cs);
-            qt[threadIdx.x] = make_double2(cs, sn);
+            qt[threadIdx.x] = unit_power(A.gamma, (double)icreg[threadIdx.x]);
         }
         if (INTW) load_phase_tables(A, smtab, threadIdx.x, kColThreads);
     }
