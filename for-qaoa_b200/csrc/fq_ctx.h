@@ -55,6 +55,7 @@ struct fq_ctx {
         double bytes;
     };
     bool profiling = false;
+    int polls = -1;  // limit of the kernels' bounded waits, < 0: their own
     bool chain = true;  // short passes may be launched in chains (chain_pass)
     std::vector<ProfRec> prof_pending;
     std::vector<cudaEvent_t> prof_pool;

@@ -26,7 +26,7 @@ int dispatch_costate(fq_ctx* ctx, bool integer, const PassArgs& A) {
 // One warp waits, with the bounded wait of the TMA pipelines (a shorter
 // poll bound: max_polls), on an mbarrier that nothing arrives at: the wait
 // gives up, the kernel records flag 2 and returns (fq_ctx_selftest_wait).
-__global__ void k_selftest_wait(int* err, long long max_polls) {
+__global__ void k_selftest_wait(int* err, int max_polls) {
     __shared__ __align__(8) unsigned long long bar;
     if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
@@ -36,10 +36,16 @@ __global__ void k_selftest_wait(int* err, long long max_polls) {
 
 }  // namespace fq
 
+extern "C" int fq_ctx_selftest_polls(fq_ctx* ctx, int polls) {
+    FQ_TRY(fq::validate_ctx(ctx));
+    ctx->polls = polls < 0 ? -1 : polls;
+    return FQ_OK;
+}
+
 extern "C" int fq_ctx_selftest_wait(fq_ctx* ctx) {
     using namespace fq;
     FQ_TRY(validate_ctx(ctx));
-    k_selftest_wait<<<1, 32, 0, ctx->stream>>>(ctx->err, 1ll << 16);
+    k_selftest_wait<<<1, 32, 0, ctx->stream>>>(ctx->err, 1 << 16);
     FQ_CUDA(cudaGetLastError());
     ctx->launches++;
     return FQ_OK;

@@ -278,6 +278,7 @@ PassArgs base_args(fq_ctx* ctx, void* sv, int N, const GraphPrep& g) {
     A.scale = 1.0;
     A.pf_dist = prefetch_distance();
     A.err = ctx->err;
+    A.polls = ctx->polls < 0 ? kWaitSpins : std::min(ctx->polls, kWaitSpins);
     return A;
 }
 

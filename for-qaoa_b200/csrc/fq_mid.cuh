@@ -40,12 +40,14 @@ struct MidArgs {
     double* partial;   // (2P + 1) x CTAs
     unsigned* counter; // grid barrier: arrivals, a multiple of kMidMaxCtas between launches
     int nb;
+    int polls;         // the barrier's limit (kMidPolls)
     int* err;
     double data[kMidWords];
 };
 static_assert(sizeof(MidArgs) <= 4096, "kernel parameters");
 
 constexpr int kMidMaxCtas = 128;
+constexpr int kMidPolls = 1 << 21;  // of some 0.7 us each
 constexpr int kMidTable = 4096;  // phase-table entries at most
 // `table`: entries of the job's phase tables.
 __host__ __device__ constexpr size_t mid_smem_bytes(int nb, bool grad, int table) {
@@ -67,7 +69,7 @@ __device__ __forceinline__ bool mid_barrier(const MidArgs& a, unsigned target) {
         ok = 0;
         __threadfence();
         atomicAdd(a.counter, 1u);
-        for (int i = 0; i < (1 << 21); i++) {
+        for (int i = 0; i < a.polls; i++) {
             unsigned c;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(a.counter) : "memory");
             if ((int)(c - target) >= 0) {

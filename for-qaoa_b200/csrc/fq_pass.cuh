@@ -132,6 +132,7 @@ struct PassArgs {
     const void* img;
     const double2* qt;
     int* err;        // device error flag (bounded waits that gave up)
+    int polls;       // their limit (kWaitSpins)
     int mir;         // mirror pass of a half state (k_pass, k_pass_dual with MIR)
     int full;        // write both halves of the state (ST = 2)
     int chained;     // 1: first pass of a chain, 2: follows the pass before it (chain_pass)

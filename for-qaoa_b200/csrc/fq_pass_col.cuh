@@ -173,6 +173,8 @@ __global__ void __launch_bounds__(kColThreads, 1)
     using SM = ColSmem<WT>;
     unsigned long long* const full = reinterpret_cast<unsigned long long*>(sm + SM::bar);
     int* const ndone = reinterpret_cast<int*>(full + kColBars);  // warps done with a stage
+    volatile int* const last = ndone + kColStages;  // the last tile loaded on each barrier, -1: none
+    volatile int* const gave_up = last + kColBars;
     WT* const kring = reinterpret_cast<WT*>(sm + SM::kp);
     WT* const creg = reinterpret_cast<WT*>(sm + SM::creg);
     WT* const cthr = reinterpret_cast<WT*>(sm + SM::cthr);
@@ -190,7 +192,11 @@ __global__ void __launch_bounds__(kColThreads, 1)
     };
 
     if (threadIdx.x == 0) {
-        for (int b = 0; b < kColBars; b++) mbar_init(&full[b], 1);
+        for (int b = 0; b < kColBars; b++) {
+            mbar_init(&full[b], 1);
+            last[b] = -1;
+        }
+        *gave_up = 0;
         for (int s = 0; s < kColStages; s++) ndone[s] = 0;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -220,6 +226,7 @@ __global__ void __launch_bounds__(kColThreads, 1)
         const int lo = T & ((1 << nmid) - 1), hi = T >> nmid;
         unsigned long long* const bar = &full[j % kColBars];
         constexpr unsigned kb = kTcutStride * sizeof(WT);
+        last[j % kColBars] = j;
         mbar_expect_tx(bar, kTileBytes + kb);
         bulk_load(kring + (j % kColBars) * kTcutStride,
                   reinterpret_cast<const WT*>(A.tcut) + (i64)T * kTcutStride, kb, bar);
@@ -240,14 +247,10 @@ __global__ void __launch_bounds__(kColThreads, 1)
     for (int j = grp; j < count; j += 2) {
         const int T = tile_of(j), s = j % kColStages;
         double2* const st = stage + (size_t)s * kTile;
-        if (!mbar_wait_bounded(&full[j % kColBars], (unsigned)((j / kColBars) & 1))) {
-            // Record it, and wait (bounded) for the copy of the group's next tile,
-            // which may be in flight; the other group waits for its own.
+        if (!mbar_wait_polls(&full[j % kColBars], (unsigned)((j / kColBars) & 1), A.polls)) {
             if (lane == 0) {
                 *(volatile int*)A.err = 1;
-                if (j + 2 < count)
-                    mbar_wait_bounded(&full[(j + 2) % kColBars],
-                                      (unsigned)(((j + 2) / kColBars) & 1));
+                *gave_up = 1;
             }
             break;
         }
@@ -334,6 +337,22 @@ __global__ void __launch_bounds__(kColThreads, 1)
         __syncwarp();
     }
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    // After a wait that gave up, copies may be in flight, and the other group
+    // may have started more: once no warp starts any, wait (bounded) for all of
+    // them, so that none lands in shared memory that is no longer this CTA's.
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned char* at = smraw;
+        asm volatile("" : "+l"(at));  // the addresses are not held across the tile loop
+        at = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(at) + 1023) &
+                                              ~(uintptr_t)1023);
+        unsigned long long* const bars = reinterpret_cast<unsigned long long*>(at + SM::bar);
+        volatile int* const loaded = reinterpret_cast<int*>(bars + kColBars) + kColStages;
+        if (loaded[kColBars])  // gave_up
+            for (int b = 0; b < kColBars; b++)
+                if (loaded[b] >= 0)
+                    mbar_wait_bounded(&bars[b], (unsigned)((loaded[b] / kColBars) & 1));
+    }
 }
 
 }  // namespace fq

@@ -29,7 +29,7 @@ constexpr unsigned kTileBytes = kTile * sizeof(double2);  // 64 KB
 // Bound on mbarrier polls: a poll that finds the phase incomplete suspends
 // the thread for ~4 us on B200 (2^16 polls measured 0.26 s), so 2^18 polls
 // give up after about a second; a landing copy ends the wait at once.
-constexpr long long kWaitSpins = 1ll << 18;
+constexpr int kWaitSpins = 1 << 18;
 
 // Box geometry of a pass (host-chosen, see make_pass_tmap):
 //   TG_CONTIG  l = 12: rank 3, box {16 doubles, 256 rows, 2}
@@ -73,8 +73,8 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
 // %globaltimer bound in the loop cost the strided pass 10% (7.05 vs 6.41 ms
 // at N=30), so the bound is a poll count.
 __device__ __forceinline__ bool mbar_wait_polls(unsigned long long* bar, unsigned parity,
-                                                long long max_polls) {
-    for (long long i = 0; i < max_polls; i++)
+                                                int max_polls) {
+    for (int i = 0; i < max_polls; i++)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kPassThreads, 1)
             issue(j + kStages - 1);
         }
         if (CUT) ct.tile(kp, base | A.goff, nF, l, a, warp, lane);  // warps 0 and 1, while the copy lands
-        if (!mbar_wait_bounded(&full[s], (unsigned)((j / kStages) & 1))) {
+        if (!mbar_wait_polls(&full[s], (unsigned)((j / kStages) & 1), A.polls)) {
             *s_abort = 1;
             if (A.err) *(volatile int*)A.err = 1;  // host memory
         }

@@ -138,6 +138,7 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
     a.partial = ctx->d_partial;
     a.counter = ctx->d_counter;
     a.err = ctx->err;
+    a.polls = ctx->polls < 0 ? kMidPolls : std::min(ctx->polls, kMidPolls);
     const void* fn = grad ? (const void*)k_mid<true> : (const void*)k_mid<false>;
     // Only the tables the job has: instances of other lanes fit beside it.
     const size_t smem = mid_smem_bytes(nb, grad, a.job.ntab * (a.job.keep ? P : 1));

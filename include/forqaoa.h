@@ -62,6 +62,11 @@ int fq_ctx_synchronize(fq_ctx* ctx);
  * fq_ctx_synchronize) returns FQ_ERR_TIMEOUT and clears the flag, and the
  * context stays usable. */
 int fq_ctx_selftest_wait(fq_ctx* ctx);
+/* The same for the waits inside the circuits' kernels: sets their limit for
+ * the context's later launches, in polls.  0: they give up at once, and a call
+ * that has such waits ends with FQ_ERR_TIMEOUT; negative: the library's own
+ * limits. */
+int fq_ctx_selftest_polls(fq_ctx* ctx, int polls);
 void* fq_ctx_stream(fq_ctx* ctx);
 /* Number of library kernels this context has launched so far. */
 int fq_ctx_kernel_launches(fq_ctx* ctx, long long* count);
