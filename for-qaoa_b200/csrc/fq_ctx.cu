@@ -263,12 +263,12 @@ int fq_ctx_create(int device, void* stream, fq_ctx** out) {
             cudaMalloc(&c->d_ptab, sizeof(double2) * kMaxPhaseTable) != cudaSuccess ||
             cudaMalloc(&c->d_partial, sizeof(double) * c->partial_cap) != cudaSuccess ||
             cudaMalloc(&c->d_tcut, kTcutBytes) != cudaSuccess ||
-            cudaMalloc(&c->d_img, kMaxGeoms * kImgStride) != cudaSuccess ||
-            cudaMalloc(&c->d_job, sizeof(double) * kJobWords) != cudaSuccess ||
-            cudaMalloc(&c->d_counter, sizeof(unsigned)) != cudaSuccess) {
+            cudaMalloc(&c->d_img, kMaxGeoms * kImgStride + sizeof(unsigned)) != cudaSuccess ||
+            cudaMalloc(&c->d_job, sizeof(double) * kJobWords) != cudaSuccess) {
             st = FQ_ERR_OOM;
             break;
         }
+        c->d_counter = (unsigned*)(c->d_img + kMaxGeoms * kImgStride);
         c->tcut_bytes = kTcutBytes;
         c->job_words = kJobWords;
         c->h_stage_bytes = std::max(wbytes, (size_t)256 * 1024);
@@ -305,7 +305,6 @@ int fq_ctx_destroy(fq_ctx* c) {
     cudaFree(c->d_partial);
     cudaFree(c->d_tcut);
     cudaFree(c->d_img);
-    cudaFree(c->d_counter);
     cudaFree(c->d_job);
     for (void* p : c->retired) cudaFree(p);
     if (c->h_stage) cudaFreeHost(c->h_stage);

@@ -27,7 +27,7 @@ struct fq_ctx {
     size_t tcut_bytes = 0;
     long long tcut_version = -1;  // g_version the tables were built for (-1: none)
     int tcut_n = -1;              // and N
-    unsigned* d_counter = nullptr;   // grid barrier of k_mid: arrivals so far
+    unsigned* d_counter = nullptr;   // grid barrier of k_mid: arrivals so far (behind d_img)
     bool cooperative = false;        // the device takes cooperative launches
     unsigned char* d_img = nullptr;  // static cut tables of the plan's geometries, built with them
     int partial_cap = 0;
