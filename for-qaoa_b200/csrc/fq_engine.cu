@@ -689,7 +689,7 @@ int fq_qaoa_forward(fq_ctx* ctx, void* sv, int N, int P, const double* graph,
     if (mid_ok(ctx, N, P)) {
         FQ_TRY(prep_graph(graph, N, g));
         FQ_TRY(run_mid(ctx, g, P, gammas, betas, SJ_STATE, (double2*)sv, nullptr, ctx->result));
-        return energy ? read_result(ctx, energy) : FQ_OK;
+        if (mid_ok(ctx, N, P)) return energy ? read_result(ctx, energy) : FQ_OK;
     }
     FQ_TRY(setup_graph(ctx, graph, N, g));
     return engine_forward(ctx, sv, N, P, g, gammas, betas, energy);

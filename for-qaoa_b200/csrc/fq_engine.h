@@ -99,6 +99,8 @@ int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, cons
               int flags, double2* state, double* out);
 // One whole circuit or gradient (SJ_STATE or SJ_GRAD) of 16..19 qubits as a
 // cooperative launch (fq_mid.cuh), where mid_ok says so; results as run_small's.
+// Nothing was launched if mid_ok says otherwise afterwards (a stream with too
+// few SMs).
 bool mid_ok(const fq_ctx* ctx, int N, int P);
 int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
             int flags, double2* state, double2* lam, double* out);

@@ -68,8 +68,9 @@ int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const doubl
     FQ_CHECK(1 + P + P * npass < kResultWords, FQ_ERR_INVALID, "P=%d too large", P);
     if (mid_ok(ctx, N, P)) {
         FQ_TRY(prep_graph(graph, N, g));
-        return run_mid(ctx, g, P, gammas, betas, SJ_GRAD, (double2*)sv, (double2*)costate,
-                       ctx->result);
+        FQ_TRY(run_mid(ctx, g, P, gammas, betas, SJ_GRAD, (double2*)sv, (double2*)costate,
+                       ctx->result));
+        if (mid_ok(ctx, N, P)) return FQ_OK;
     }
     FQ_TRY(setup_graph(ctx, graph, N, g));
 

@@ -147,9 +147,16 @@ int run_mid(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const 
                                  (int)mid_smem_bytes(kMidMaxBits, grad, kMidTable)));
     void* args[1] = {&a};
     const int tok = prof_begin(ctx);
-    FQ_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem,
-                                        ctx->stream));
+    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem,
+                                                      ctx->stream);
     prof_end(ctx, tok, FQ_KIND_OTHER, 0.0);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        // The stream has fewer SMs than the device: the passes from now on.
+        cudaGetLastError();
+        ctx->cooperative = false;
+        return FQ_OK;
+    }
+    FQ_CUDA(e);
     ctx->launches++;
     return FQ_OK;
 }

@@ -19,7 +19,7 @@ static pthread_mutex_t mu = PTHREAD_MUTEX_INITIALIZER;
 static char text[1 << 20];
 static size_t used;
 static struct { const void* fn; const char* name; } kernels[4096];
-static int nkernels, capture, capture_mode, query;
+static int nkernels, capture, capture_mode, query, cooperative;
 static __thread config pushed;
 
 static void note(const char* fmt, ...) {
@@ -40,7 +40,8 @@ static int launch(const void* fn, void** args) {
     return OK;
 }
 
-/* For the test: the log so far (emptied), event queries' status, capture. */
+/* For the test: the log so far (emptied), the status of event queries and of
+ * cooperative launches, capture. */
 size_t fake_log(char* out, size_t n) {
     pthread_mutex_lock(&mu);
     const size_t k = used < n ? used : n;
@@ -51,6 +52,7 @@ size_t fake_log(char* out, size_t n) {
 }
 void fake_event_query(int status) { query = status; }
 void fake_capture(int on) { capture = on; }
+void fake_cooperative(int status) { cooperative = status; }
 
 /* Registration and launches. */
 void** __cudaRegisterFatBinary(void* p) { static void* h; (void)p; return &h; }
@@ -78,7 +80,7 @@ int cudaLaunchKernel(const void* fn, dim g, dim b, void** a, size_t m, void* s) 
 }
 int cudaLaunchCooperativeKernel(const void* fn, dim g, dim b, void** a, size_t m, void* s) {
     (void)g, (void)b, (void)m, (void)s;
-    return launch(fn, a);
+    return cooperative ? cooperative : launch(fn, a);
 }
 int cudaLaunchKernelExC(const void* cfg, const void* fn, void** a) {
     (void)cfg;

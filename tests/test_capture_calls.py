@@ -1,5 +1,6 @@
 """CPU tests, over a CUDA runtime without a device, of what calls under
-stream capture leave to the graph and what is done at once."""
+stream capture leave to the graph and what is done at once, and of what runs
+where a cooperative launch is refused."""
 import fake_cuda
 
 BARRIER = """
@@ -95,3 +96,26 @@ print("ok")
 
 def test_captured_circuits_carry_weights_and_tables(tmp_path):
     assert "ok" in fake_cuda.run(TABLES, tmp_path)
+
+
+PARTITION = """
+ctx = fq.Context(0)
+st, cs = ctx.state(18), ctx.state(18)
+def circuit():
+    log()
+    ctx.qaoa_forward(st, graph(18), [0.1, 0.2], [0.3, 0.4], energy=False)
+    return log()
+assert [x for x in circuit() if "k_mid" in x]
+fake.fake_cooperative(720)  # the launch is too large for what the stream has
+for _ in range(2):
+    out = circuit()
+    assert any("k_pass" in x for x in out) and not any("k_mid" in x for x in out), out
+with fq.Context(0) as c:
+    c.energy_grad(18, graph(18), [0.1], [0.3], st, cs)
+    assert any("k_pass_dual" in x for x in log())
+print("ok")
+"""
+
+
+def test_streams_with_few_sms_run_the_passes(tmp_path):
+    assert "ok" in fake_cuda.run(PARTITION, tmp_path)

@@ -10,7 +10,7 @@ from conftest import angles, assert_state_close, complete_int
 pytestmark = pytest.mark.gpu
 
 
-# 16, 19: a grid barrier (32 CTAs, 128 CTAs of another tile size); 24, 26: TMA
+# 16, 19: a grid barrier (64 CTAs, 128 CTAs of another tile size); 24, 26: TMA
 # pipelines, of warps and of CTAs.
 @pytest.mark.parametrize("n", [16, 19, 24, 26])
 def test_waits_give_up_and_later_circuits_are_right(fq, oracle, n):
