@@ -202,14 +202,16 @@ static int choose_lrows(int N) {
 // rows when fewer qubits remain).  The first pass of a layer carries its
 // cost phase (layer 0: the launch-control init), and the fused schedule
 // runs the first and last passes of consecutive layers as one sweep, so
-// with three or more passes the contiguous pass (four exchanges when fused,
-// two alone) goes second and never fuses: on B200 at N=30, p=5, 59.5-59.7
-// layers/s against 57.2-57.6 with it first (A/B in one call).  The strided
-// passes over the highest qubits lead and the one over the lowest closes
-// each layer: an odd circuit then ends on the faster of the two strided
-// geometries (61.2-61.8 against 60.3-61.0 layers/s, A/B in one call).
+// with three or more passes the contiguous or mirror pass (four exchanges
+// when fused, two alone) goes second and never fuses.  The strided passes
+// over the highest qubits lead and the one over the lowest closes each layer.
 // A half state's passes cover the same number of qubits: the mirror tile
 // takes qubits 0..10 and N-1, the strided ones 11..N-2.
+// Circuits on half states on B200, three runs in turn in one call, ms:
+//                            N=28 p=3     N=30 p=4     N=30 p=5   N=32 p=3 (FP64)
+//   this order                5.39-5.40    31.8-32.1    37.9-38.2    124-125
+//   mirror pass first         5.92-5.93    33.5-34.0    42.7-43.0    160-161
+//   lowest strided one first  5.47-5.49    31.0-31.8    38.7-39.1    132
 std::vector<PassPlan> plan_layer(int N, bool half) {
     std::vector<PassPlan> v;
     if (half)

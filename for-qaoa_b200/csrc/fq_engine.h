@@ -78,9 +78,10 @@ bool engine_fused(const GraphPrep& g, int P);
 int engine_last_pass(const GraphPrep& g, int N, int P);
 int chain_pass(const fq_ctx* ctx, i64 ntiles, int per_sm, bool first);
 
-// The gradient of more than kSmallJobMaxQubits qubits split for asynchronous use: grad_enqueue puts every
-// kernel and the final device-to-host copy of the results on ctx's stream;
-// once the stream has passed that point, grad_collect assembles them.
+// The gradient of more than kSmallJobMaxQubits qubits split for asynchronous
+// use: grad_enqueue puts every kernel on ctx's stream, the last of which write
+// the results to ctx->result (pinned); once the stream has passed that point,
+// and without an error, grad_collect assembles them.
 int grad_enqueue(fq_ctx* ctx, void* sv, void* costate, int N, int P, const double* graph,
                  const double* gammas, const double* betas);
 int grad_collect(fq_ctx* ctx, int N, int P, double* energy, double* grad_gamma,

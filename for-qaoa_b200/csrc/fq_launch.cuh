@@ -35,15 +35,14 @@ inline double pass_bytes(const PassArgs& A) {
                 (EX == EX_COSTATE ? 16.0 : 0.0));
 }
 
-// Strided tiles with 128-byte rows run as paired CTAs (k_pass with PAIR:
-// the two tiles that differ in physical bit 3 at once, so DRAM sees 256-byte
-// rows).  Measured on B200 at N=30, p=5 (A/B in one call): 59.8-60.1
-// layers/s with every such pass paired, 59.5-59.7 with the strided RX pass
-// on the TMA pipeline instead.
-// Strided tiles with rows of 2, 4 or 8 amplitudes run paired (k_pass PAIR):
-// rows of 16 and more are DRAM-friendly alone.  Rows of 2 and 4 (N = 23,
-// 22, 32) paired: 0.527 against 0.542 ms per N=23 circuit (p=5), 233
-// against 242 ms per N=32 circuit (p=3), A/B in one call.
+// Strided tiles with rows of 2, 4 or 8 amplitudes run as paired CTAs (k_pass
+// with PAIR: the two tiles that differ in physical bit l at once, so DRAM sees
+// rows twice as long); rows of 16 and more are DRAM-friendly alone.
+// Circuits on half states on B200, paired against not, three runs in turn in
+// one call: rows of 4, N=23 p=5 0.319 / 0.327 ms, with FP64 weights 0.337 /
+// 0.351, N=32 p=3 124 / 126 ms; rows of 8, N=30 p=5 37.9-38.2 / 38.1-38.4 ms
+// (the first and the last strided pass; the fused ones are k_pass_col's); rows
+// of 2, N=22 p=5 0.160 / 0.159, no difference.
 inline bool pair_ok(const PassArgs& A) { return A.l >= 1 && A.l <= 3 && A.a > A.l && A.ntiles >= 2; }
 
 constexpr size_t kSoloSmem = 120 * 1024;  // more than half an SM's shared memory
@@ -121,8 +120,8 @@ inline PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
 // over strided tiles with rows of 16 or more amplitudes.  Contiguous tiles
 // and tiles with 128-byte rows (paired) run on k_pass, whose per-thread
 // loads from two CTAs per SM measured faster there on B200 at N=30 (the
-// contiguous RX pass: 6.0 ms against 6.9 ms on the TMA pipeline); passes
-// with a phase always do.
+// contiguous RX pass over a whole state: 6.0 ms against 6.9 ms on the TMA
+// pipeline); passes with a phase always do.
 inline bool tma_for(int ph, const PassArgs& A) {
     return ph == PH_NONE && A.l >= 4 && A.l < kTileBits && !A.mir;
 }

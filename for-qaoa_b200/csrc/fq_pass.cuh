@@ -44,6 +44,8 @@
 // amplitudes, one walked backwards).  Phases, cut constants and rotations
 // see an ordinary tile of the N-qubit state.  The pass that ends a forward
 // circuit writes both halves (ST = 2).  Measured: engine_args, fq_engine.h.
+// Times of single passes at N=30 quoted below for a choice of the pass's own
+// code are those of whole-state sweeps, twice a half state's.
 //
 // Cut value of an amplitude (exact in integers for integer weights):
 //   C(z) = K(fixed) + C_TT(tile bits) + sum_{u in tile} z_u e_u(fixed)
@@ -1016,11 +1018,14 @@ __global__ void __launch_bounds__(PAIR ? 2 * kPassThreads : kPassThreads, PAIR ?
         }
         if (!PAIR && LOAD && A.pf_dist > 0 && (contiguous || MIR)) {
             // Stream this CTA's tile pf_dist strides ahead from HBM into L2
-            // (one bulk prefetch).  Strided tiles are not prefetched: per-
-            // thread row prefetches cost more than they saved (12.2 against
-            // 11.2 ms on the fused strided pass at N=30), and so did a tensor
-            // prefetch of the tile as a TMA box (61.5 against 58.1-61.0
-            // layers/s at N=30, p=5; A/B in one call).
+            // (one bulk prefetch; a mirror tile's two runs).  Circuits on half
+            // states on B200, three runs in turn in one call, distance 1 / 0
+            // (off) / 2: N=30 p=5 37.9-38.2 / 39.5-39.8 / 38.5-38.8 ms, N=28
+            // p=3 5.39-5.40 / 5.72-5.74 / 5.54-5.57, N=23 no difference.
+            // Strided tiles are not prefetched: on whole states per-thread row
+            // prefetches cost more than they saved (12.2 against 11.2 ms on
+            // the fused strided pass at N=30), and so did a tensor prefetch of
+            // the tile as a TMA box (58.1-61.0 against 61.5 layers/s).
             const i64 T2 = T + (i64)A.pf_dist * gridDim.x;
             if (T2 < A.ntiles && tid < (MIR ? 2 : 1)) {
                 i64 b2 = ((T2 & ((1ll << nmid) - 1)) << l) |

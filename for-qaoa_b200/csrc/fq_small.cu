@@ -115,9 +115,9 @@ int launch_small_batch(const SmallJob* jobs, int njobs, int c, cudaStream_t st) 
     return launch_any<true>(c, nullptr, jobs, njobs, st);
 }
 
-// Amplitude bits per CTA: 128 CTAs, as small as two warps.  On B200, gradient
-// p=6 with 9, 10, 11, 12 bits: N=16 107, 117, 141, 189 us; N=18 124
-// with 10, 150, 202; N=19 148 with 11, 206 with 12.
+// Amplitude bits per CTA: 128 CTAs (64 at N=16), as small as two warps.  On
+// B200, gradient p=6, integer weights, with 9, 10, 11, 12 bits: N=16 107, 117,
+// 141, 189 us; N=18 124 with 10, 150, 202; N=19 148 with 11, 206 with 12.
 static int mid_bits(int N) { return std::max(kMidMinBits, N - 8); }
 
 bool mid_ok(const fq_ctx* ctx, int N, int P) {

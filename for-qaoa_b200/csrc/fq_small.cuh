@@ -166,7 +166,7 @@ struct SmallLay {
 };
 
 // One instance on one CTA (CB = 0, run-time nb) or on a cluster of 2^CB
-// CTAs (nb = 11).  blockDim.x may exceed the 2^(nb-4) threads that hold
+// CTAs (nb = 11).  blockDim.x may exceed the 2^(nb-3) threads that hold
 // amplitudes: the others help to fill the phase tables.
 template <bool GRAD, int CB>
 struct SmallRun {
