@@ -418,7 +418,8 @@ int setup_graph(fq_ctx* ctx, const double* graph, int N, GraphPrep& g) {
 
 // The tables of a circuit's pass geometries that depend on the graph alone,
 // built by one launch (k_tile_cuts) and kept while the weights and N stay
-// the same: every tile's cut constants in ctx->d_tcut (grown on demand,
+// the same (upload_graph; a new graph costs 11 to 20 us a call on B200, upload
+// and launch): every tile's cut constants in ctx->d_tcut (grown on demand,
 // tabs[i] serves plan[i]; null when it cannot be had, the passes then
 // compute them per tile) and the static tables of each geometry in
 // ctx->d_img.  The tile constants are 64 B per tile (128 B with FP64
@@ -426,7 +427,7 @@ int setup_graph(fq_ctx* ctx, const double* graph, int N, GraphPrep& g) {
 // work on two warps and the barrier after it.  The images replace each
 // CTA's own set-up from the weights, a chain of dependent shared-memory
 // reads and sincos before its first tile, which at one tile per CTA was half
-// of a pass.  On B200 (A/B in one call): forward N=20 p=5 112 against 140 us
+// of a pass.  On B200 (calls on one graph, A/B in one call): forward N=20 p=5 112 against 140 us
 // with the set-up in every pass, N=23 p=4 (FP64 weights) 291 against 315 us;
 // gradient N=19 p=6 215 against 279 us; N >= 26 within 1%.
 static int tile_cut_tables(fq_ctx* ctx, const GraphPrep& g, int N,

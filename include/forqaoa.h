@@ -48,9 +48,14 @@ int fq_version(void);
 /* ---- context ------------------------------------------------------------
  * One context per (device, stream).  It owns the small device scratch used
  * by the kernels (weights, phase tables, reduction partials) and pinned
- * staging memory, allocated once at creation.  stream == NULL creates a
+ * staging memory, allocated once at creation; only per-tile tables (from 25
+ * qubits on) and the data of circuits of up to 15 qubits and more than 2048
+ * layers outgrow it.  stream == NULL creates a
  * private non-blocking stream (the reference's compute_stream,
- * src/state.cpp:139). */
+ * src/state.cpp:139).
+ * A circuit without *energy can be captured in a CUDA graph.  The graph holds
+ * the graph's weights and the angles, uses the context's scratch, and may be
+ * replayed between the context's calls, as long as the context lives. */
 int fq_ctx_create(int device, void* stream, fq_ctx** out);
 int fq_ctx_destroy(fq_ctx* ctx);
 int fq_ctx_synchronize(fq_ctx* ctx);

@@ -98,3 +98,25 @@ def test_replays_between_calls_on_other_graphs(fq, oracle, n, P):
         finally:
             st.free()
             st25.free()
+
+
+def test_tables_grow_during_a_capture(fq):
+    """The first call, captured, is of a size whose tables outgrow the
+    context's: its replay gives the state of the call that follows."""
+    n, P = 25, 2
+    rng = np.random.default_rng(n)
+    W, (g, b) = complete_int(n, rng), angles(rng, P)
+    stream, ctx = context(fq)
+    with ctx as c:
+        st = c.state(n)
+        try:
+            cap = Captured(c, stream, st, W, g, b)
+            c.qaoa_forward(st, W, g, b, energy=False)
+            want = st.to_host()
+            st.init_basis0()
+            c.synchronize()
+            cap.replay()
+            assert np.array_equal(st.to_host(), want)
+            assert abs(np.linalg.norm(want) - 1) <= 1e-12
+        finally:
+            st.free()
