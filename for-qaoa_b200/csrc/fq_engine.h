@@ -98,6 +98,11 @@ void small_job(const GraphPrep& g, int P, const double* gammas, const double* be
 // else 1) and state (SJ_STATE) are device-accessible.
 int run_small(fq_ctx* ctx, const GraphPrep& g, int P, const double* gammas, const double* betas,
               int flags, double2* state, double* out);
+// run_small's launch of size class c >= 4, one instance or njobs descriptors on
+// the device.
+struct SmallArgs;
+int launch_small_cluster(int c, bool grad, const SmallArgs* one, const SmallJob* jobs, int njobs,
+                         cudaStream_t stream);
 // One whole circuit or gradient (SJ_STATE or SJ_GRAD) of 16..19 qubits as a
 // cooperative launch (fq_mid.cuh), where mid_ok says so; results as run_small's.
 // Nothing was launched if mid_ok says otherwise afterwards (a stream with too
