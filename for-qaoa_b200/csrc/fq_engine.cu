@@ -363,9 +363,9 @@ void set_table_args(PassArgs& A, const GraphPrep& g, double gamma, double scale)
         A.ntab = (int)(dhi - dlo + 1);
         // exp(-i*gamma*W/2), turned by the product's rounding error (unit_power).
         const double W = (double)g.W_int, x = gamma * W, lo = fma(gamma, W, -x) / 2;
-        const double c = cos(x / 2), s = sin(x / 2);
-        A.ph0x = scale * (c - s * lo);
-        A.ph0y = -scale * (s + c * lo);
+        const double c = cos(x / 2), s = sin(x / 2), cl = cos(lo), sl = sin(lo);
+        A.ph0x = scale * (c * cl - s * sl);
+        A.ph0y = -scale * (s * cl + c * sl);
     }
 }
 

@@ -173,9 +173,10 @@ static_assert(kTableStride * kMaxTableLayers <= kMaxPhaseTable, "layer tables fi
 // to 1.2e-13 -> 1e-14 of their largest entry.
 __device__ __forceinline__ double2 unit_power(double g, double v) {
     const double x = __dmul_rn(g, v), lo = fma(g, v, -x);
-    double sn, cs;
+    double sn, cs, sl = lo, cl = 1.0;
     sincos(x, &sn, &cs);
-    return make_double2(fma(-lo, sn, cs), fma(lo, cs, sn));
+    if (!(fabs(lo) <= 1e-8)) sincos(lo, &sl, &cl);  // x beyond 2^26
+    return make_double2(fma(-sl, sn, cs * cl), fma(sl, cs, sn * cl));
 }
 
 // Shared-memory bytes reserved for the two-level phase table.

@@ -84,3 +84,29 @@ def test_integer_phases_are_as_exact_as_the_rotations(ctx, seed):
     assert abs(float(got - e)) <= TOL * float(e) and abs(float(e2 - e)) <= TOL * float(e)
     assert float(np.abs(db - gb).max()) <= TOL * float(e)
     assert float(np.abs(dg - gg).max()) <= TOL * float(e)
+
+
+@pytest.mark.parametrize("gamma", [3e7, -4e9, 3.7e12, 1e18, 1e30])
+def test_large_angles(ctx, gamma):
+    """Far beyond 2^26 the rounding of gamma * C is no small angle: the
+    phases are those of the exact product (11 and 53 bits: long double holds
+    it) and the norm is kept."""
+    n = 20
+    rng = np.random.default_rng(n)
+    W, b = complete_int(n, rng), 0.7
+    z = np.arange(1 << n)
+    cut = np.zeros(1 << n, dtype=np.int64)
+    for i in range(n):
+        for j in range(i + 1, n):
+            cut += int(W[i, j]) * (((z >> i) ^ (z >> j)) & 1)
+    v = [np.full(1 << n, np.sqrt(LD(2)) ** -n), np.zeros(1 << n, dtype=LD)]
+    phase(v, cut, W.sum(), gamma)
+    for q in range(n):
+        rotate(v, q, b)
+    st = ctx.state(n)
+    try:
+        ctx.qaoa_forward(st, W, [gamma], [b])
+        psi = st.to_host()
+    finally:
+        st.free()
+    assert float(np.sqrt(((psi.real - v[0]) ** 2 + (psi.imag - v[1]) ** 2).sum())) <= TOL / 2
